@@ -22,6 +22,9 @@ cudaError_t rbmpp_launch_sampler(const DevDims&, const DevTables&, const DevPara
                                  cudaStream_t);
 size_t rbmpp_sampler_smem(const DevDims&, int);
 int rbmpp_stream_stages(const DevDims&, int);
+int rbmpp_resident_threads(const DevDims&, int);
+cudaError_t rbmpp_launch_sampler_resident(const DevDims&, const DevTables&, const DevParams&, const DevWalkers&, int, int,
+                                          cudaStream_t);
 cudaError_t rbmpp_launch_sampler_stream(const DevDims&, const DevTables&, const DevParams&, const DevWalkers&, int, int,
                                         cudaStream_t);
 cudaError_t rbmpp_launch_estimator(const DevDims&, const DevTables&, const DevParams&, const int8_t*, int, double*,
@@ -179,6 +182,7 @@ struct rbmpp_ctx {
   cudaEvent_t ev[12] = {};
   double stats[10] = {0};
   int stream_stages = 0;  // > 0: TMA-streamed sampler with this many stages
+  bool sampler_auto = true;  // RBMPP_SAMPLER did not choose the direct sampler
   bool est_fits = true;   // the estimator's workspace fits in shared memory (tiles there or in global scratch)
   bool est_smem_tiles = true;  // ... with its tiles in shared memory
   double* d_SE = nullptr;  // Slater_Elm [qp][2N][2N] of the skew form (transverse projection)
@@ -424,6 +428,16 @@ int check_walker_status(rbmpp_ctx* c, const int* d_status, int n, const char* wh
   return 0;
 }
 
+// Threads per block when the context samples with its inverse blocks resident in shared memory, else 0.  A walker
+// that fits is latency-bound and several times faster there than streamed or read from L2 (figures in
+// sampler_resident.cuh).  The verification hooks address the streaming sampler's pipeline, so they keep it.
+int resident_threads(const rbmpp_ctx* c) {
+  if (!c->sampler_auto || c->d.skip_load > 0 || c->d.wait_polls > 0) return 0;
+  int maxsm = 0;
+  if (cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->dims.device) != cudaSuccess) return 0;
+  return rbmpp_resident_threads(c->d, maxsm);
+}
+
 }  // namespace
 
 // ===================================================================================================
@@ -496,7 +510,10 @@ int rbmpp_create(const rbmpp_dims* dims, rbmpp_ctx** out) {
   c->est_fits = (long long)rbmpp_estimator_smem_any(d, maxsm) <= maxsm;
   c->est_smem_tiles = (long long)rbmpp_estimator_smem(d, 256) <= maxsm;
   c->stream_stages = rbmpp_stream_stages(d, maxsm);
-  if (getenv("RBMPP_SAMPLER") && std::string(getenv("RBMPP_SAMPLER")) == "direct") c->stream_stages = 0;
+  if (getenv("RBMPP_SAMPLER") && std::string(getenv("RBMPP_SAMPLER")) == "direct") {
+    c->stream_stages = 0;
+    c->sampler_auto = false;
+  }
   if (d.alphac) c->stream_stages = 0;  // the streaming sampler carries real units only
   int r;
   const int N = d.N;
@@ -773,6 +790,8 @@ int rbmpp_make_sample(rbmpp_ctx* c, int first, int* naccept, long long* naccept_
   CK(cudaEventRecord(c->ev[0], c->st));
   if (c->d.skew)
     CK(rbmpp_launch_sampler_skew(c->d, tables(c), params(c), c->W, first ? 1 : 0, c->st));
+  else if (const int rt = resident_threads(c))
+    CK(rbmpp_launch_sampler_resident(c->d, tables(c), params(c), c->W, first ? 1 : 0, rt, c->st));
   else if (c->stream_stages > 0)
     CK(rbmpp_launch_sampler_stream(c->d, tables(c), params(c), c->W, first ? 1 : 0, c->stream_stages, c->st));
   else
@@ -1573,12 +1592,16 @@ int rbmpp_get_stats(const rbmpp_ctx* c, double* out, int n) {
 
 // ===================================================================================================
 // Batched make_sample: several contexts (lattice sizes, couplings, parameter sets) on one device sampled
-// by one persistent launch of the direct sampler, with the launch shape and the walker order chosen by a
-// measuring autotuner.
+// together, with the launch shape and the walker order chosen by a measuring autotuner: one persistent launch for the
+// contexts whose walkers are resident in shared memory, and beside it one of the direct sampler for the others.
 // ===================================================================================================
 cudaError_t rbmpp_launch_sampler_batch(const BatchInst*, const int2*, int, int, int, int, size_t, long long*,
                                        cudaStream_t);
 int rbmpp_batch_occupancy(int, int, size_t);
+int rbmpp_resident_batch_threads(const DevDims&);
+size_t rbmpp_resident_smem(const DevDims&, int);
+cudaError_t rbmpp_launch_resident_batch(const BatchInst*, const int2*, int, int, int, size_t, long long*, cudaStream_t);
+int rbmpp_resident_batch_occupancy(int, size_t);
 
 struct rbmpp_batch {
   std::vector<rbmpp_ctx*> ctx;
@@ -1586,6 +1609,13 @@ struct rbmpp_batch {
   int total = 0, kpl = 1, threads = 256, order = 0, nsm = 0;
   size_t smem[3] = {0, 0, 0};  // dynamic shared memory for 128, 256, 512 threads
   std::vector<double> cost;    // per-walker cost of each context (model, then measured)
+  // contexts whose walkers are resident in shared memory go in a launch of their own, beside the direct sampler's
+  std::vector<char> res;       // 1: resident
+  int n_direct = 0;            // blocks of the direct launch: the first entries of the schedule
+  int res_threads = 0;
+  size_t res_smem = 0;
+  cudaStream_t st2 = nullptr;
+  cudaEvent_t join = nullptr;
   BatchInst* d_inst = nullptr;
   int2* d_sched = nullptr;
   long long* d_cycles = nullptr;
@@ -1640,6 +1670,7 @@ std::vector<int2> make_schedule(const rbmpp_batch* b, int order) {
         if (w < b->ctx[k]->d.nw) s.push_back(make_int2(k, w));
     std::stable_sort(s.begin(), s.end(), [&](const int2& a, const int2& c2) { return b->cost[a.x] > b->cost[c2.x]; });
   }
+  std::stable_partition(s.begin(), s.end(), [&](const int2& a) { return !b->res[a.x]; });
   return s;
 }
 
@@ -1651,6 +1682,22 @@ double makespan(const std::vector<int2>& sched, const std::vector<double>& cost,
     *it += cost[j.x];
   }
   return *std::max_element(load.begin(), load.end());
+}
+
+// The launches of one schedule of n blocks, nd of them direct, on st (the resident ones on the batch's second
+// stream, which st waits for).
+cudaError_t launch_batch(rbmpp_batch* b, int n, int nd, int first, int threads, size_t smem, long long* cycles,
+                         cudaStream_t st) {
+  cudaError_t e = cudaSuccess;
+  if (nd > 0)
+    e = rbmpp_launch_sampler_batch(b->d_inst, b->d_sched, nd, first, b->kpl, threads, smem, cycles, st);
+  if (!e && n > nd) {
+    e = rbmpp_launch_resident_batch(b->d_inst, b->d_sched + nd, n - nd, first, b->res_threads, b->res_smem,
+                                    cycles ? cycles + nd : nullptr, b->st2);
+    if (!e) e = cudaEventRecord(b->join, b->st2);
+    if (!e) e = cudaStreamWaitEvent(st, b->join, 0);
+  }
+  return e;
 }
 
 int upload_insts(rbmpp_batch* b, const std::vector<DevDims>* dims_override) {
@@ -1687,7 +1734,13 @@ int rbmpp_batch_create(rbmpp_ctx* const* ctxs, int n, rbmpp_batch** out) {
     b->ctx.push_back(c);
     b->off.push_back(b->total);
     b->total += c->d.nw;
-    b->kpl = std::max(b->kpl, (c->d.Np + 31) / 32);
+    b->res.push_back(resident_threads(c) > 0);
+    if (b->res[k]) {
+      b->res_threads = std::max(b->res_threads, rbmpp_resident_batch_threads(c->d));
+    } else {
+      b->n_direct += c->d.nw;
+      b->kpl = std::max(b->kpl, (c->d.Np + 31) / 32);
+    }
     // cost model until measured: proposals x (Y bytes read per proposal + the per-proposal fixed work)
     const double sweeps = (double)(c->d.nwarm + c->d.ns + 1);
     b->cost.push_back(sweeps * c->d.N * ((double)c->d.n_qp * c->d.Np * c->d.Np + 64.0 * c->d.N));
@@ -1695,6 +1748,20 @@ int rbmpp_batch_create(rbmpp_ctx* const* ctxs, int n, rbmpp_batch** out) {
   BCK(cudaSetDevice(dev));
   int maxsm = 0;
   BCK(cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  // a context whose own block shape fits shared memory may not at the batch's: it goes with the direct ones
+  for (int k = 0; k < n; k++)
+    if (b->res[k]) {
+      const size_t need = rbmpp_resident_smem(ctxs[k]->d, b->res_threads);
+      if ((long long)need + 4096 > maxsm) {  // and the batched kernel's static shared memory
+        b->res[k] = 0;
+        b->n_direct += ctxs[k]->d.nw;
+        b->kpl = std::max(b->kpl, (ctxs[k]->d.Np + 31) / 32);
+      } else {
+        b->res_smem = std::max(b->res_smem, need);
+      }
+    }
+  BCK(cudaStreamCreateWithFlags(&b->st2, cudaStreamNonBlocking));
+  BCK(cudaEventCreateWithFlags(&b->join, cudaEventDisableTiming));
   BCK(cudaDeviceGetAttribute(&b->nsm, cudaDevAttrMultiProcessorCount, dev));
   const int opts[3] = {128, 256, 512};
   for (int i = 0; i < 3; i++) {
@@ -1721,6 +1788,8 @@ int rbmpp_batch_destroy(rbmpp_batch* b) {
   if (b->d_cycles) cudaFree(b->d_cycles);
   for (auto& e : b->ev)
     if (e) cudaEventDestroy(e);
+  if (b->join) cudaEventDestroy(b->join);
+  if (b->st2) cudaStreamDestroy(b->st2);
   delete b;
   return 0;
 }
@@ -1743,6 +1812,8 @@ int rbmpp_batch_tune(rbmpp_batch* b, int* threads_out, int* order_out, double* p
     pd[k].ns = 0;
     for (int w = 0; w < std::min(8, b->ctx[k]->d.nw); w++) probe.push_back(make_int2(k, w));
   }
+  const auto split = std::stable_partition(probe.begin(), probe.end(), [&](const int2& a) { return !b->res[a.x]; });
+  const int pnd = (int)(split - probe.begin());
   // the probed walkers' random streams and Nfastup are saved and restored
   std::vector<std::vector<uint32_t>> mt(n);
   std::vector<std::vector<int>> nf(n);
@@ -1764,11 +1835,12 @@ int rbmpp_batch_tune(rbmpp_batch* b, int* threads_out, int* order_out, double* p
   std::vector<double> best_cost = b->cost;
   for (int i = 0; i < 3; i++) {
     if (!b->smem[i]) continue;
-    const int occ = rbmpp_batch_occupancy(b->kpl, opts[i], b->smem[i]);
+    if (pnd == 0 && opts[i] != b->threads) continue;  // the block size concerns the direct launch only
+    const int occ = pnd ? rbmpp_batch_occupancy(b->kpl, opts[i], b->smem[i])
+                        : rbmpp_resident_batch_occupancy(b->res_threads, b->res_smem);
     if (occ < 1) continue;
     BCK(cudaEventRecord(b->ev[0], st));
-    BCK(rbmpp_launch_sampler_batch(b->d_inst, b->d_sched, (int)probe.size(), 1, b->kpl, opts[i], b->smem[i],
-                                   b->d_cycles, st));
+    BCK(launch_batch(b, (int)probe.size(), pnd, 1, opts[i], b->smem[i], b->d_cycles, st));
     BCK(cudaEventRecord(b->ev[1], st));
     BCK(cudaStreamSynchronize(st));
     float ms = 0.f;
@@ -1827,8 +1899,7 @@ int rbmpp_batch_make_sample(rbmpp_batch* b, int first, long long* naccept_total)
   cudaStream_t st = b->ctx[0]->st;
   const int ti = thr_index(b->threads);
   BCK(cudaEventRecord(b->ev[0], st));
-  BCK(rbmpp_launch_sampler_batch(b->d_inst, b->d_sched, b->total, first ? 1 : 0, b->kpl, b->threads, b->smem[ti],
-                                 nullptr, st));
+  BCK(launch_batch(b, b->total, b->n_direct, first ? 1 : 0, b->threads, b->smem[ti], nullptr, st));
   BCK(cudaEventRecord(b->ev[1], st));
   BCK(cudaStreamSynchronize(st));
   float ms = 0.f;
