@@ -718,6 +718,9 @@ int rbmpp_set_tables(rbmpp_ctx* c, const int* W_map, const double* para, const i
   for (int k = 0; k < d.n_slater; k++)
     if (cnt[k] > 1) inj = 0;
   c->d.orb_injective = inj;
+  c->d.orb_identity = d.n_slater == N * N;
+  for (int k = 0; k < N * N && c->d.orb_identity; k++)
+    if (c->orb_host[k] != k) c->d.orb_identity = 0;
   CK(cudaMemcpy(c->d_wmap, wmap.data(), sizeof(int) * wmap.size(), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(c->d_winv, winv.data(), sizeof(int) * winv.size(), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(c->d_para, para, sizeof(double) * 2 * d.n_mp, cudaMemcpyHostToDevice));

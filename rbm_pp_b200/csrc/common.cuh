@@ -27,6 +27,7 @@ struct DevDims {
   int alphac, Mc;     // complex RBM units (RBM.f90 thetac): Mc = 2 alphac n_mp complex angles, kept after the
                       //   Mr real ones in every theta array as (re, im) pairs
   int nw, ns, nupdate, nwarm;
+  int orb_identity;   // Orbital_Idx(p, q) = p N + q (0-based): the full map, which needs no look-up
   int orb_injective;  // Orbital_Idx is injective within each spin block for one projection
   int pf_sign;        // (-1)^{Np(Np-1)/2}
   int gj_global;      // the direct sampler's Gauss-Jordan tile lives in DevWalkers::gj (too large for SMEM)
