@@ -9,14 +9,65 @@ void rbmpp_note_launch();  // capi.cu: counts kernel launches
 
 namespace {
 
-// C(i, j) = alpha * sum_k A(k, i) B(k, j) + beta * C(i, j) on upper-triangular 128 x 128 tiles.
-// A(k, i) = A[k * sk + i * si] (same for B).  KCONTIG selects the coalesced load direction.
-constexpr int BM = 128, BK = 8, TM = 8;
+// C(i, j) = alpha * sum_k A(k, i) A(k, j) (+ C(i, j) with ACC) for i <= j, on upper-triangular BM x BM tiles of the FP64
+// matrix units.  A(k, i) = A[k * sk + i * si]: KCONTIG has sk = 1 (the Cholesky's trailing update), else si = 1
+// (S = O^T O).
+//
+// Bound by the FP64 pipe (37 TFLOP/s by mma.m8n8k4.f64, measured; 33 by FMA).  At BM = 128 eight warps hold 64 x 32
+// accumulators each (32 pieces of 8 x 8), so a step of four k costs twelve shared loads for 32 products; operands come
+// by cp.async into kStages buffers.  Both operands are kept as [k][i] (row length 4 mod 16) or, with KCONTIG, [i][k]
+// (likewise), which puts an 8 x 4 fragment on distinct banks either way.  VEC = 2: 16-byte copies, for a base and a
+// stride of whole 16-byte words; an odd stride takes 8-byte ones.
+// Measured against the form before (FMA, 8 x 8 results a thread, loads one step ahead): the S build of 8192 samples x
+// 4226 parameters 13.2 -> 5.8 ms, factorisation and solve of 10404 parameters 56.3 -> 34.3 ms.
+constexpr int BK = 16, kStages = 4, kLdK = BK + 4;
 
-template <bool KCONTIG>
-__global__ void __launch_bounds__(256) gemm_atb_upper(int n, int K, const double* __restrict__ A, long long sk,
-                                                      long long si, double alpha, double beta, double* __restrict__ C,
-                                                      long long ldc, int row0) {
+template <int BM, bool KCONTIG>
+constexpr int kTileDoubles = KCONTIG ? BM * kLdK : BK * (BM + 4);
+template <int BM, bool KCONTIG>
+constexpr int kGemmSmem = kStages * 2 * kTileDoubles<BM, KCONTIG> * 8;
+
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, int bytes) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async8(void* dst, const void* src, int bytes) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+}
+
+// One operand tile: k0 .. k0 + BK of columns i0 .. i0 + BM; zeros beyond K and n
+template <int BM, bool KCONTIG, int VEC>
+__device__ __forceinline__ void load_operand(double* dst, const double* __restrict__ A, long long sk, long long si,
+                                             int n, int K, int i0, int k0) {
+  constexpr int kWords = BM * BK / VEC;
+#pragma unroll
+  for (int r = 0; r < kWords / 256; r++) {
+    const int e = threadIdx.x + 256 * r;
+    int kk, ii, left;
+    double* d;
+    if (KCONTIG) {
+      kk = (e % (BK / VEC)) * VEC;
+      ii = e / (BK / VEC);
+      left = i0 + ii < n ? K - (k0 + kk) : 0;
+      d = dst + ii * kLdK + kk;
+    } else {
+      ii = (e % (BM / VEC)) * VEC;
+      kk = e / (BM / VEC);
+      left = k0 + kk < K ? n - (i0 + ii) : 0;
+      d = dst + kk * (BM + 4) + ii;
+    }
+    const int cnt = left <= 0 ? 0 : left < VEC ? left : VEC;
+    const double* src = cnt ? A + (long long)(k0 + kk) * sk + (long long)(i0 + ii) * si : A;
+    if (VEC == 2) cp_async16(d, src, 8 * cnt);
+    else cp_async8(d, src, 8 * cnt);
+  }
+}
+
+template <int BM, bool KCONTIG, bool ACC, int VEC>
+__global__ void __launch_bounds__(256, BM > 64 ? 1 : 2) gemm_atb_upper(int n, int K, const double* __restrict__ A, long long sk,
+                                                         long long si, double alpha, double* __restrict__ C,
+                                                         long long ldc, int row0) {
   // upper-tile index -> (ti, tj) with ti <= tj
   const int nt = (n - row0 + BM - 1) / BM;
   int t = blockIdx.x, ti = 0;
@@ -26,66 +77,107 @@ __global__ void __launch_bounds__(256) gemm_atb_upper(int n, int K, const double
   }
   const int tj = ti + t;
   const int i0 = row0 + ti * BM, j0 = row0 + tj * BM;
-  __shared__ double As[2][BK][BM];
-  __shared__ double Bs[2][BK][BM];
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  double acc[TM][TM];
+  extern __shared__ __align__(16) double sm[];
+  constexpr int TD = kTileDoubles<BM, KCONTIG>, kLdI = BM + 4, PI = BM / 16, PJ = BM / 32;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, c = lane & 3;
+  const int wi = (warp & 1) * (BM / 2), wj = (warp >> 1) * (BM / 4);  // the warp's part
+  double acc[PI][PJ][2];
 #pragma unroll
-  for (int a = 0; a < TM; a++)
+  for (int a = 0; a < PI; a++)
 #pragma unroll
-    for (int b = 0; b < TM; b++) acc[a][b] = 0.0;
-
-  auto load = [&](int buf, int k0) {
-#pragma unroll
-    for (int r = 0; r < (BK * BM) / 256; r++) {
-      int e = tid + 256 * r;
-      int kk, ii;
-      if (KCONTIG) {
-        kk = e % BK;
-        ii = e / BK;
-      } else {
-        kk = e / BM;
-        ii = e % BM;
-      }
-      int k = k0 + kk;
-      int ia = i0 + ii, jb = j0 + ii;
-      As[buf][kk][ii] = (k < K && ia < n) ? A[(long long)k * sk + (long long)ia * si] : 0.0;
-      Bs[buf][kk][ii] = (k < K && jb < n) ? A[(long long)k * sk + (long long)jb * si] : 0.0;
+    for (int b = 0; b < PJ; b++) acc[a][b][0] = acc[a][b][1] = 0.0;
+  const int steps = (K + BK - 1) / BK;
+  auto load = [&](int st) {
+    if (st < steps) {
+      double* p = sm + (st % kStages) * 2 * TD;
+      load_operand<BM, KCONTIG, VEC>(p, A, sk, si, n, K, i0, st * BK);
+      load_operand<BM, KCONTIG, VEC>(p + TD, A, sk, si, n, K, j0, st * BK);
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  load(0, 0);
-  __syncthreads();
-  int buf = 0;
-  for (int k0 = 0; k0 < K; k0 += BK) {
-    if (k0 + BK < K) load(buf ^ 1, k0 + BK);
 #pragma unroll
-    for (int kk = 0; kk < BK; kk++) {
-      double a[TM], b[TM];
+  for (int st = 0; st < kStages - 1; st++) load(st);
+  for (int st = 0; st < steps; st++) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
+    __syncthreads();  // step st has landed everywhere, and everybody is done with the buffer refilled below
+    load(st + kStages - 1);
+    const double* As = sm + (st % kStages) * 2 * TD;
+    const double* Bs = As + TD;
 #pragma unroll
-      for (int m = 0; m < TM; m++) {
-        a[m] = As[buf][kk][tx + 16 * m];
-        b[m] = Bs[buf][kk][ty + 16 * m];
+    for (int k = 0; k < BK; k += 4) {
+      double fa[PI], fb[PJ];
+#pragma unroll
+      for (int a = 0; a < PI; a++)
+        fa[a] = KCONTIG ? As[(wi + 8 * a + g) * kLdK + k + c] : As[(k + c) * kLdI + wi + 8 * a + g];
+#pragma unroll
+      for (int b = 0; b < PJ; b++)
+        fb[b] = KCONTIG ? Bs[(wj + 8 * b + g) * kLdK + k + c] : Bs[(k + c) * kLdI + wj + 8 * b + g];
+#pragma unroll
+      for (int a = 0; a < PI; a++)
+#pragma unroll
+        for (int b = 0; b < PJ; b++)
+          asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+              : "+d"(acc[a][b][0]), "+d"(acc[a][b][1])
+              : "d"(fa[a]), "d"(fb[b]));
+    }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll
+  for (int b = 0; b < PJ; b++)
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      const int j = j0 + wj + 8 * b + 2 * c + e;
+      if (j >= n) continue;
+      double* col = C + ldc * j;
+      double old[PI];
+      if (ACC) {
+#pragma unroll
+        for (int a = 0; a < PI; a++) {
+          const int i = i0 + wi + 8 * a + g;
+          old[a] = i <= j ? col[i] : 0.0;
+        }
       }
 #pragma unroll
-      for (int p = 0; p < TM; p++)
-#pragma unroll
-        for (int q = 0; q < TM; q++) acc[p][q] = fma(a[p], b[q], acc[p][q]);
+      for (int a = 0; a < PI; a++) {
+        const int i = i0 + wi + 8 * a + g;
+        if (i <= j) col[i] = ACC ? old[a] + alpha * acc[a][b][e] : alpha * acc[a][b][e];
+      }
     }
-    __syncthreads();
-    buf ^= 1;
-  }
-#pragma unroll
-  for (int q = 0; q < TM; q++) {
-    int j = j0 + ty + 16 * q;
-    if (j >= n) continue;
-#pragma unroll
-    for (int p = 0; p < TM; p++) {
-      int i = i0 + tx + 16 * p;
-      if (i >= n || i > j) continue;
-      double* c = C + (long long)i + ldc * j;
-      *c = (beta == 0.0) ? alpha * acc[p][q] : beta * (*c) + alpha * acc[p][q];
-    }
-  }
+}
+
+template <int BM, bool KCONTIG, bool ACC>
+cudaError_t launch_gemm_bm(int n, int K, const double* A, long long sk, long long si, double alpha, double* C,
+                           long long ldc, int row0, cudaStream_t st) {
+  const int nt = (n - row0 + BM - 1) / BM;
+  const long long stride = KCONTIG ? si : sk;
+  const bool vec = stride % 2 == 0 && (uintptr_t)A % 16 == 0 && row0 % 2 == 0;
+  auto* f = vec ? gemm_atb_upper<BM, KCONTIG, ACC, 2> : gemm_atb_upper<BM, KCONTIG, ACC, 1>;
+  cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem<BM, KCONTIG>);
+  if (e != cudaSuccess) return e;
+  rbmpp_note_launch();
+  f<<<nt * (nt + 1) / 2, 256, kGemmSmem<BM, KCONTIG>, st>>>(n, K, A, sk, si, alpha, C, ldc, row0);
+  return cudaGetLastError();
+}
+
+// The tile size with the least time by waves of whole tiles: a wave of 96-wide tiles takes 0.6 of one of 128-wide ones
+// (0.56 of the products, at slightly more loads for each), two 64-wide tiles to an SM 0.6 too (half the products, at
+// twice the loads).  A last wave that is nearly empty (595 tiles of 128 at 4226 rows: four waves and three tiles)
+// or a matrix of few tiles is what the smaller sizes are for.
+template <bool KCONTIG, bool ACC>
+cudaError_t launch_gemm_atb_upper(int n, int K, const double* A, long long sk, long long si, double alpha, double* C,
+                                  long long ldc, int row0, cudaStream_t st) {
+  int dev = 0, nsm = 1;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return e;
+  auto waves = [&](int bm, int slots) {
+    const long long nt = (n - row0 + bm - 1) / bm, tiles = nt * (nt + 1) / 2;
+    return (double)((tiles + slots - 1) / slots);
+  };
+  const double t128 = waves(128, nsm), t96 = 0.6 * waves(96, nsm), t64 = 0.6 * waves(64, 2 * nsm);
+  if (t128 <= t96 && t128 <= t64) return launch_gemm_bm<128, KCONTIG, ACC>(n, K, A, sk, si, alpha, C, ldc, row0, st);
+  if (t96 <= t64) return launch_gemm_bm<96, KCONTIG, ACC>(n, K, A, sk, si, alpha, C, ldc, row0, st);
+  return launch_gemm_bm<64, KCONTIG, ACC>(n, K, A, sk, si, alpha, C, ldc, row0, st);
 }
 
 // mirror the upper triangle into the lower one
@@ -269,11 +361,7 @@ __global__ void sample_scalars_kernel(int ns, const double* psi, int psi_stride,
 // host wrappers
 // ------------------------------------------------------------------------------------------------
 cudaError_t rbmpp_syrk_ot_o(int nv, int ns, const double* O, double* S, cudaStream_t st) {
-  int nt = (nv + BM - 1) / BM;
-  int ntiles = nt * (nt + 1) / 2;
-  rbmpp_note_launch();
-  gemm_atb_upper<false><<<ntiles, 256, 0, st>>>(nv, ns, O, nv, 1, 1.0, 0.0, S, nv, 0);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_gemm_atb_upper<false, false>(nv, ns, O, nv, 1, 1.0, S, nv, 0, st);
   if (e) return e;
   dim3 g((nv + 31) / 32, (nv + 31) / 32);
   rbmpp_note_launch();
@@ -284,10 +372,8 @@ cudaError_t rbmpp_syrk_ot_o(int nv, int ns, const double* O, double* S, cudaStre
 // C(i, j) = sum_k A(k, i) A(k, j) for i <= j (upper triangle, column-major C), A(k, i) = A[k sk + i si]
 cudaError_t rbmpp_gemm_atb_upper(int n, int K, const double* A, long long sk, long long si, double* C, long long ldc,
                                  cudaStream_t st) {
-  int nt = (n + BM - 1) / BM;
-  rbmpp_note_launch();
-  gemm_atb_upper<false><<<nt * (nt + 1) / 2, 256, 0, st>>>(n, K, A, sk, si, 1.0, 0.0, C, ldc, 0);
-  return cudaGetLastError();
+  if (si != 1) return cudaErrorInvalidValue;
+  return launch_gemm_atb_upper<false, false>(n, K, A, sk, 1, 1.0, C, ldc, 0, st);
 }
 
 cudaError_t rbmpp_symmetrize(int n, double* S, cudaStream_t st) {
@@ -301,12 +387,9 @@ cudaError_t rbmpp_symmetrize(int n, double* S, cudaStream_t st) {
 // update of the blocked Cholesky in sr_solve.cu; K = its panel width, A(k, i) contiguous in k)
 cudaError_t rbmpp_gemm_atb_upper_acc(int n, int K, const double* A, long long sk, long long si, double alpha,
                                      double* C, long long ldc, int row0, cudaStream_t st) {
-  const int rest = n - row0;
-  if (rest <= 0) return cudaSuccess;
-  const int nt = (rest + BM - 1) / BM;
-  rbmpp_note_launch();
-  gemm_atb_upper<true><<<nt * (nt + 1) / 2, 256, 0, st>>>(n, K, A, sk, si, alpha, 1.0, C, ldc, row0);
-  return cudaGetLastError();
+  if (n - row0 <= 0) return cudaSuccess;
+  if (sk != 1) return cudaErrorInvalidValue;
+  return launch_gemm_atb_upper<true, true>(n, K, A, 1, si, alpha, C, ldc, row0, st);
 }
 
 cudaError_t rbmpp_trmv_upper(int n, const double* A, const double* x, double* y, cudaStream_t st) {
