@@ -26,12 +26,26 @@ namespace {
 
 constexpr int kSkThreads = 256;
 constexpr int kSkWarps = kSkThreads / 32;
+// The sampler's largest block: a proposal reads every G of the walker from L2 or HBM, so it wants as many warps with
+// rows in flight as the registers allow (half as many where their workspaces do not fit).
+constexpr int kSmpThreads = 512;
+// The sampler's kernels take N = L^2 as a template argument (even L, so 4, 16, 36, 64 and 100 are all there are): the
+// inner loops lose most of their address and bounds arithmetic.  Measured against a run-time N, make_sample of 64
+// walkers without translations: 6.2 -> 5.5 ms at 4x4, 12.5 -> 10.5 at 6x6, 36.2 -> 23.4 at 8x8; 8 walkers at 10x10:
+// 111 -> 91 ms.
+// Rows of G in flight per warp (a warp's row is (N + 31) / 32 loads a lane) in a pass that reads G, and in one that
+// also writes it.  One row pair at a time paid an L2 round trip for every two rows of every projection.
+constexpr int kpl(int N) { return (N + 31) / 32; }
+constexpr int rows_read(int N) { return N == 36 ? 12 : N == 100 ? 10 : 16; }
+constexpr int rows_update(int N) { return N == 36 ? 6 : N == 100 ? 5 : 8; }
 
 __device__ __forceinline__ int rho_of(const int* idx, int e, int Np, int N) { return idx[e] + (e >= Np ? N : 0); }
 
 // row r of Slater_Elm for projection qp: SE(r, .)
-__device__ __forceinline__ const double* se_row(const DevDims& d, const DevParams& p, int qp, int r) {
-  return p.SE + ((size_t)qp * 2 * d.N + r) * 2 * (size_t)d.N;
+template <int N>
+__device__ __forceinline__ const double* se_row(const DevParams& p, int qp, int r) {
+  constexpr int N2 = 2 * N;
+  return p.SE + (size_t)(qp * N2 + r) * N2;
 }
 
 // update_slater_elements, slater.f90:7-64, all four blocks: row site rj, column site ri,
@@ -59,20 +73,29 @@ __global__ void build_se_kernel(int N, int n_mp, const int* wmap, const int* orb
 }
 
 // B(i, j) = -SE(rho_i, rho_j) into a warp tile (ld = N + 1)
-__device__ __forceinline__ void warp_gather_skew(double* T, const DevDims& d, const DevParams& p, int qp,
-                                                 const int* idx) {
-  const int N = d.N, Np = d.Np, ld = N + 1, lane = threadIdx.x & 31;
-  for (int i = 0; i < N; i++) {
-    const double* row = se_row(d, p, qp, rho_of(idx, i, Np, N));
-    for (int j = lane; j < N; j += 32) T[i * ld + j] = -row[rho_of(idx, j, Np, N)];
+template <int N>
+__device__ __forceinline__ void warp_gather_skew(double* T, const DevParams& p, int qp, const int* idx) {
+  constexpr int Np = N / 2, ld = N + 1, B = N < 18 ? N : N == 100 ? 10 : N == 64 ? 16 : 18;
+  const int lane = threadIdx.x & 31;
+  for (int j = lane; j < N; j += 32) {
+    const int rj = rho_of(idx, j, Np, N);
+#pragma unroll 1
+    for (int i0 = 0; i0 < N; i0 += B) {  // B loads in flight
+      double v[B];
+#pragma unroll
+      for (int i = 0; i < B; i++) v[i] = se_row<N>(p, qp, rho_of(idx, i0 + i, Np, N))[rj];
+#pragma unroll
+      for (int i = 0; i < B; i++) T[(i0 + i) * ld + j] = -v[i];
+    }
   }
   __syncwarp();
 }
 
 // Pf(T) by Parlett-Reid elimination with row/column pivoting; T (n x n, ld = n + 1) is destroyed.
-template <int KPL>
-__device__ double warp_pfaffian(double* T, int n, bool& singular) {
-  const int ld = n + 1, lane = threadIdx.x & 31;
+template <int n>
+__device__ double warp_pfaffian(double* T, bool& singular) {
+  constexpr int ld = n + 1, KPL = kpl(n);
+  const int lane = threadIdx.x & 31;
   double pf = 1.0;
   singular = false;
   for (int k = 0; k + 1 < n; k += 2) {
@@ -126,14 +149,17 @@ __device__ double warp_pfaffian(double* T, int n, bool& singular) {
         rr[m] = in ? T[(k + 1) * ld + j] : 0.0;
       }
       __syncwarp();
-      for (int i = k + 2; i < n; i++) {
-        const double ti = T[i * ld + k] / piv, ri = T[(k + 1) * ld + i];
 #pragma unroll
-        for (int m = 0; m < KPL; m++) {
-          const int j = lane + 32 * m;
-          if (j >= k + 2 && j < n) T[i * ld + j] = fma(ri, tau[m], fma(-ti, rr[m], T[i * ld + j]));
+      for (int mi = 0; mi < KPL; mi++)
+#pragma unroll 4
+        for (int i = max(k + 2, 32 * mi); i < min(n, 32 * mi + 32); i++) {
+          const double ti = __shfl_sync(0xffffffffu, tau[mi], i & 31), ri = __shfl_sync(0xffffffffu, rr[mi], i & 31);
+#pragma unroll
+          for (int m = 0; m < KPL; m++) {
+            const int j = lane + 32 * m;
+            if (j >= k + 2 && j < n) T[i * ld + j] = fma(ri, tau[m], fma(-ti, rr[m], T[i * ld + j]));
+          }
         }
-      }
       __syncwarp();
     }
   }
@@ -143,9 +169,10 @@ __device__ double warp_pfaffian(double* T, int n, bool& singular) {
 // G = (B^-1 - B^-T) / 2 in place (matrix.f90:96-105) from warp_gj's inverse, whose column j sits at perm[j].
 // The symmetric part of the computed inverse is rounding noise, which the exchange-ratio formula would amplify
 // by the conditioning of B; the skew part alone gives ratios to about 1e-13.
-template <int KPL>
-__device__ void warp_unpermute_skew(double* T, int n, const int* perm) {
-  const int ld = n + 1, lane = threadIdx.x & 31;
+template <int n>
+__device__ void warp_unpermute_skew(double* T, const int* perm) {
+  constexpr int ld = n + 1, KPL = kpl(n);
+  const int lane = threadIdx.x & 31;
   for (int i = 0; i < n; i++) {
     double v[KPL];
 #pragma unroll
@@ -175,12 +202,12 @@ __device__ void warp_unpermute_skew(double* T, int n, const int* perm) {
 // calculate_MAll for the skew form (policy of the walker routines of sampler_common.cuh): one warp per
 // projection on its own shared-memory tile; writes G (when write_y) and pf_out; with diff, the drift measure
 // of make_sample.f90:106-113 against the stored G.
-template <int KPL>
+template <int N>
 struct SkewScratch {
   static __device__ void run(const SCtx& c, const int* idx, double* pf_out, bool write_y, bool diff) {
     const DevDims& d = c.d;
     const WS& s = c.s;
-    const int N = d.N, ld = N + 1;
+    constexpr int ld = N + 1, KPL = kpl(N);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     double wratio = -1.0;
     int bad = 0;  // 1: singular, 2: inverse not skew (matrix.f90:103)
@@ -188,12 +215,12 @@ struct SkewScratch {
       double* T = c.par_tiles + (size_t)warp * N * ld;
       int* perm = (int*)(s.wS + (size_t)warp * d.Np);
       for (int qp = warp; qp < d.n_qp && !bad; qp += c.par_ntile) {
-        warp_gather_skew(T, d, c.p, qp, idx);
+        warp_gather_skew<N>(T, c.p, qp, idx);
         bool sing;
-        const double pfq = warp_pfaffian<KPL>(T, N, sing);
+        const double pfq = warp_pfaffian<N>(T, sing);
         if (!sing) {
-          warp_gather_skew(T, d, c.p, qp, idx);
-          (void)warp_gj<KPL, 0, 4>(T, N, perm, sing);
+          warp_gather_skew<N>(T, c.p, qp, idx);
+          (void)warp_gj<KPL, N, 4>(T, N, perm, sing);
         }
         if (sing) {
           bad = 1;
@@ -241,9 +268,12 @@ struct SkewScratch {
 };
 
 // x^_i = B'(i, a) = SE(rho'_a, rho_i) and y^_i = SE(rho'_b, rho_i) (skew Slater_Elm), zero at i = a, b
-__device__ __forceinline__ void warp_gather_xy(const DevDims& d, const double* SEa, const double* SEb, const int* idx,
+template <int N>
+__device__ __forceinline__ void warp_gather_xy(const double* SEa, const double* SEb, const int* idx,
                                                int a, int b, double* xh, double* yh) {
-  const int N = d.N, Np = d.Np, lane = threadIdx.x & 31;
+  constexpr int Np = N / 2;
+  const int lane = threadIdx.x & 31;
+#pragma unroll 4
   for (int i = lane; i < N; i += 32) {
     const int ri = rho_of(idx, i, Np, N);
     const bool ab = i == a || i == b;
@@ -254,40 +284,35 @@ __device__ __forceinline__ void warp_gather_xy(const DevDims& d, const double* S
 }
 
 // (G x^)_j and (G y^)_j for this lane's columns j = lane + 32 m (G skew: (G v)_j = -sum_i v_i G(i, j))
-template <int KPL>
-__device__ __forceinline__ void warp_gxy(const double* Gq, int N, const double* xh, const double* yh, double (&gx)[KPL],
-                                         double (&gy)[KPL]) {
+template <int N>
+__device__ __forceinline__ void warp_gxy(const double* Gq, const double* xh, const double* yh,
+                                         double (&gx)[kpl(N)], double (&gy)[kpl(N)]) {
+  constexpr int KPL = kpl(N);
   const int lane = threadIdx.x & 31;
   double ax[KPL], ay[KPL];
 #pragma unroll
   for (int m = 0; m < KPL; m++) ax[m] = ay[m] = 0.0;
-  int i = 0;
-  for (; i + 2 <= N; i += 2) {
-    const double x0 = xh[i], y0 = yh[i], x1 = xh[i + 1], y1 = yh[i + 1];
-    double g0[KPL], g1[KPL];
+  constexpr int B = rows_read(N);
+#pragma unroll(N <= 36 ? (N + B - 1) / B : 1)
+  for (int i0 = 0; i0 < N; i0 += B) {
+    double g[B][KPL];
 #pragma unroll
-    for (int m = 0; m < KPL; m++) {
-      const int j = lane + 32 * m;
-      g0[m] = j < N ? Gq[(size_t)i * N + j] : 0.0;
-      g1[m] = j < N ? Gq[(size_t)(i + 1) * N + j] : 0.0;
-    }
+    for (int r = 0; r < B; r++)
 #pragma unroll
-    for (int m = 0; m < KPL; m++) {
-      ax[m] = fma(x1, g1[m], fma(x0, g0[m], ax[m]));
-      ay[m] = fma(y1, g1[m], fma(y0, g0[m], ay[m]));
-    }
-  }
-  for (; i < N; i++) {
-    const double x0 = xh[i], y0 = yh[i];
-#pragma unroll
-    for (int m = 0; m < KPL; m++) {
-      const int j = lane + 32 * m;
-      if (j < N) {
-        const double g = Gq[(size_t)i * N + j];
-        ax[m] = fma(x0, g, ax[m]);
-        ay[m] = fma(y0, g, ay[m]);
+      for (int m = 0; m < KPL; m++) {
+        const int j = lane + 32 * m;
+        g[r][m] = (i0 + r < N && j < N) ? Gq[(i0 + r) * N + j] : 0.0;
       }
-    }
+#pragma unroll
+    for (int r = 0; r < B; r++)
+      if (i0 + r < N) {
+        const double x = xh[i0 + r], y = yh[i0 + r];
+#pragma unroll
+        for (int m = 0; m < KPL; m++) {
+          ax[m] = fma(x, g[r][m], ax[m]);
+          ay[m] = fma(y, g[r][m], ay[m]);
+        }
+      }
   }
 #pragma unroll
   for (int m = 0; m < KPL; m++) {
@@ -296,56 +321,77 @@ __device__ __forceinline__ void warp_gxy(const double* Gq, int N, const double* 
   }
 }
 
+// One projection's G (N x N, N even) into the warp's shared buffer, asynchronously; fetch_wait before reading it.  The
+// warp that reads a projection is the one that writes it, so program order and __syncwarp order the accesses.
+template <int N>
+__device__ __forceinline__ void fetch_tile(double* buf, const double* Gq) {
+  __syncwarp();
+  const uint32_t dst = smem_u32(buf);
+#pragma unroll 4
+  for (int e = threadIdx.x & 31; e < N * N / 2; e += 32)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * e), "l"(Gq + 2 * e) : "memory");
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+__device__ __forceinline__ void fetch_wait() {
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncwarp();
+}
+
 // Pf(B') / Pf(B) for the exchange of electrons a -> rho'_a, b -> rho'_b (valid on all lanes)
-template <int KPL>
-__device__ double warp_skew_ratio(const DevDims& d, const DevParams& p, const double* Gq, int qp, const int* idx,
-                                  int a, int b, int ra_new, int rb_new, double* xh, double* yh) {
-  const int lane = threadIdx.x & 31, N = d.N;
-  const double* SEa = se_row(d, p, qp, ra_new);
-  const double* SEb = se_row(d, p, qp, rb_new);
-  warp_gather_xy(d, SEa, SEb, idx, a, b, xh, yh);
+template <int N>
+__device__ __forceinline__ double warp_skew_ratio(const DevDims& d, const DevParams& p, const double* Gq,
+                                                  int qp, const int* idx,
+                                  int a, int b, int ra_new, int rb_new, double* xh, double* yh, bool staged) {
+  constexpr int KPL = kpl(N);
+  const int lane = threadIdx.x & 31;
+  const double* SEa = se_row<N>(p, qp, ra_new);
+  const double* SEb = se_row<N>(p, qp, rb_new);
+  warp_gather_xy<N>(SEa, SEb, idx, a, b, xh, yh);
   const double ya = -SEa[rb_new];  // B'(a, b)
+  if (staged) fetch_wait();
   double gx[KPL], gy[KPL];
-  warp_gxy<KPL>(Gq, N, xh, yh, gx, gy);
+  warp_gxy<N>(Gq, xh, yh, gx, gy);
   double xgy = 0.0, gxa = 0.0, gxb = 0.0, gya = 0.0, gyb = 0.0;
 #pragma unroll
   for (int m = 0; m < KPL; m++) {
     const int j = lane + 32 * m;
     if (j < N) {
       xgy = fma(xh[j], gy[m], xgy);
-      if (j == a) {
-        gxa = gx[m];
-        gya = gy[m];
-      }
-      if (j == b) {
-        gxb = gx[m];
-        gyb = gy[m];
-      }
+    }
+    const double xa = __shfl_sync(0xffffffffu, gx[m], a & 31), xb = __shfl_sync(0xffffffffu, gx[m], b & 31);
+    const double yb = __shfl_sync(0xffffffffu, gy[m], b & 31), yc = __shfl_sync(0xffffffffu, gy[m], a & 31);
+    if (m == (a >> 5)) {
+      gxa = xa;
+      gya = yc;
+    }
+    if (m == (b >> 5)) {
+      gxb = xb;
+      gyb = yb;
     }
   }
   xgy = warp_sum(xgy);
-  gxa = warp_sum(gxa);
-  gxb = warp_sum(gxb);
-  gya = warp_sum(gya);
-  gyb = warp_sum(gyb);
   const double gab = Gq[(size_t)a * N + b];
   __syncwarp();
   return -gab * (ya + xgy) + gxa * gyb - gxb * gya;
 }
 
-// G' = G + V K^{-1} V^T after the accepted exchange; v: [4][N] per-warp scratch for the columns of V
-template <int KPL>
-__device__ void warp_skew_update(const DevDims& d, const DevParams& p, double* Gq, int qp, const int* idx, int a,
+// G' = G + V K^{-1} V^T after the accepted exchange, from Gq (global, or the warp's shared buffer) to Go (global);
+// v: [4][N] per-warp scratch for the columns of V, then the rows of V K^{-1}
+template <int N>
+__device__ __forceinline__ void warp_skew_update(const DevDims& d, const DevParams& p, const double* Gq,
+                                                 double* Go, int qp, const int* idx, int a,
                                  int b, int ra_old, int rb_old, int ra_new, int rb_new, double* xh, double* yh,
-                                 double* v) {
-  const int lane = threadIdx.x & 31, N = d.N;
-  const double* SEa = se_row(d, p, qp, ra_new);
-  const double* SEb = se_row(d, p, qp, rb_new);
-  warp_gather_xy(d, SEa, SEb, idx, a, b, xh, yh);
+                                 double* v, bool staged) {
+  constexpr int KPL = kpl(N);
+  const int lane = threadIdx.x & 31;
+  const double* SEa = se_row<N>(p, qp, ra_new);
+  const double* SEb = se_row<N>(p, qp, rb_new);
+  warp_gather_xy<N>(SEa, SEb, idx, a, b, xh, yh);
   const double xb = SEa[rb_new];                           // B'(b, a)
-  const double bab = -se_row(d, p, qp, ra_old)[rb_old];    // B(a, b) before the move
+  const double bab = -se_row<N>(p, qp, ra_old)[rb_old];    // B(a, b) before the move
+  if (staged) fetch_wait();
   double gx[KPL], gy[KPL];
-  warp_gxy<KPL>(Gq, N, xh, yh, gx, gy);
+  warp_gxy<N>(Gq, xh, yh, gx, gy);
   // V = [G dx, G e_a, G dy, G e_b]: G dx = G x^ + x_b G(:, b) - e_a, G dy = G y^ - e_b + B(a, b) G(:, a)
   double V[KPL][4];
   double v0a = 0.0, v0b = 0.0, v2a = 0.0, v2b = 0.0, xv2 = 0.0;
@@ -362,21 +408,19 @@ __device__ void warp_skew_update(const DevDims& d, const DevParams& p, double* G
 #pragma unroll
       for (int q = 0; q < 4; q++) v[q * N + j] = V[m][q];
       xv2 = fma(xh[j] + (j == b ? xb : 0.0), V[m][2], xv2);
-      if (j == a) {
-        v0a = V[m][0];
-        v2a = V[m][2];
-      }
-      if (j == b) {
-        v0b = V[m][0];
-        v2b = V[m][2];
-      }
+    }
+    const double w0a = __shfl_sync(0xffffffffu, V[m][0], a & 31), w2a = __shfl_sync(0xffffffffu, V[m][2], a & 31);
+    const double w0b = __shfl_sync(0xffffffffu, V[m][0], b & 31), w2b = __shfl_sync(0xffffffffu, V[m][2], b & 31);
+    if (m == (a >> 5)) {
+      v0a = w0a;
+      v2a = w2a;
+    }
+    if (m == (b >> 5)) {
+      v0b = w0b;
+      v2b = w2b;
     }
   }
   xv2 = warp_sum(xv2);
-  v0a = warp_sum(v0a);
-  v0b = warp_sum(v0b);
-  v2a = warp_sum(v2a);
-  v2b = warp_sum(v2b);
   const double gab = Gq[(size_t)a * N + b];
   __syncwarp();
   // K = U^T G U - J (skew): upper entries
@@ -388,38 +432,70 @@ __device__ void warp_skew_update(const DevDims& d, const DevParams& p, double* G
                            {k23 * ip, 0.0, -k03 * ip, k02 * ip},
                            {-k13 * ip, k03 * ip, 0.0, -k01 * ip},
                            {k12 * ip, -k02 * ip, k01 * ip, 0.0}};
-  for (int i = 0; i < N; i++) {
-    double z[4];
+  // rows of V K^{-1}, one row per lane, in place of the columns of V
+  double z[KPL][4];
+#pragma unroll
+  for (int m = 0; m < KPL; m++) {
+    const int i = lane + 32 * m < N ? lane + 32 * m : N - 1;
     const double vi[4] = {v[i], v[N + i], v[2 * N + i], v[3 * N + i]};
 #pragma unroll
-    for (int q = 0; q < 4; q++) z[q] = vi[0] * Ki[0][q] + vi[1] * Ki[1][q] + vi[2] * Ki[2][q] + vi[3] * Ki[3][q];
-    double* Gr = Gq + (size_t)i * N;
+    for (int q = 0; q < 4; q++) z[m][q] = vi[0] * Ki[0][q] + vi[1] * Ki[1][q] + vi[2] * Ki[2][q] + vi[3] * Ki[3][q];
+  }
+  __syncwarp();
 #pragma unroll
-    for (int m = 0; m < KPL; m++) {
-      const int j = lane + 32 * m;
-      if (j < N) {
-        double g = Gr[j];
-#pragma unroll
-        for (int q = 0; q < 4; q++) g = fma(z[q], V[m][q], g);
-        Gr[j] = g;
-      }
+  for (int m = 0; m < KPL; m++) {
+    const int i = lane + 32 * m;
+    if (i < N) {
+      *reinterpret_cast<double2*>(v + 4 * i) = make_double2(z[m][0], z[m][1]);
+      *reinterpret_cast<double2*>(v + 4 * i + 2) = make_double2(z[m][2], z[m][3]);
     }
+  }
+  __syncwarp();
+  constexpr int B = rows_update(N);
+#pragma unroll(N <= 36 ? (N + B - 1) / B : 1)
+  for (int i0 = 0; i0 < N; i0 += B) {
+    double g[B][KPL];
+#pragma unroll
+    for (int r = 0; r < B; r++)
+#pragma unroll
+      for (int m = 0; m < KPL; m++) {
+        const int j = lane + 32 * m;
+        g[r][m] = (i0 + r < N && j < N) ? Gq[(i0 + r) * N + j] : 0.0;
+      }
+#pragma unroll
+    for (int r = 0; r < B; r++)
+      if (i0 + r < N) {
+        const int i = i0 + r;
+        const double2 za = *reinterpret_cast<const double2*>(v + 4 * i),
+                      zb = *reinterpret_cast<const double2*>(v + 4 * i + 2);
+#pragma unroll
+        for (int m = 0; m < KPL; m++) {
+          const int j = lane + 32 * m;
+          if (j < N)
+            Go[i * N + j] = fma(zb.y, V[m][3], fma(zb.x, V[m][2], fma(za.y, V[m][1], fma(za.x, V[m][0], g[r][m]))));
+        }
+      }
   }
   __syncwarp();
 }
 
 // Shared memory of the skew sampler: the walker workspace, 6 N doubles per warp (x^, y^, the columns of V),
 // and ntile from-scratch tiles of N x (N + 1) doubles.
-__host__ __device__ size_t skew_sampler_smem(const DevDims& d, int ntile, size_t* vec_off, size_t* tile_off) {
-  size_t off = ws_layout(d, kSkWarps, nullptr, nullptr, false);
+__host__ __device__ size_t skew_sampler_smem(const DevDims& d, int nwarps, int ntile, size_t* vec_off,
+                                             size_t* tile_off) {
+  size_t off = ws_layout(d, nwarps, nullptr, nullptr, false);
   if (vec_off) *vec_off = off;
-  off = align16(off + (size_t)kSkWarps * 6 * d.N * 8);
+  off = align16(off + (size_t)nwarps * 6 * d.N * 8);
   if (tile_off) *tile_off = off;
   return off + (size_t)ntile * d.N * (d.N + 1) * 8;
 }
 
-template <int KPL>
-__global__ void __launch_bounds__(kSkThreads, 1)
+// Bounded by instructions on the SMs that have a walker: with the walker's G in L2 (72 projections of 10 KB at 6x6) a
+// proposal is an x^ . G y^ product per projection, 2,800 warp instructions each before N was a constant.  Measured,
+// make_sample of 64 walkers, 6x6 with translations, 35 sweeps: 104 -> 65 ms with 16 warps, row batches and staged
+// fetches (8 warps, two rows in flight, straight from L2), -> 49 ms with N a constant.
+template <int N>
+__global__ void __launch_bounds__(kSmpThreads, 1)
     sampler_skew_kernel(const __grid_constant__ DevDims d, const __grid_constant__ DevTables t,
                         const __grid_constant__ DevParams p, const __grid_constant__ DevWalkers W, int first,
                         int ntile) {
@@ -428,17 +504,24 @@ __global__ void __launch_bounds__(kSkThreads, 1)
   const int w = blockIdx.x;
   if (w >= d.nw) return;
   size_t vec_off = 0, tile_off = 0;
-  skew_sampler_smem(d, ntile, &vec_off, &tile_off);
-  if (threadIdx.x == 0) ws_layout(d, kSkWarps, smem, &ws, false);
+  skew_sampler_smem(d, blockDim.x >> 5, ntile, &vec_off, &tile_off);
+  if (threadIdx.x == 0) ws_layout(d, blockDim.x >> 5, smem, &ws, false);
   __syncthreads();
-  const int N = d.N, Np = d.Np;
+  constexpr int Np = N / 2;
   const SCtx c{d, t, p, W, w, ws, W.Y + (size_t)w * d.n_qp * N * N, (double*)(smem + tile_off), ntile};
   const WS& s = ws;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nwarps = blockDim.x >> 5;
   double* xh = (double*)(smem + vec_off) + (size_t)warp * 6 * N;
   double* yh = xh + N;
   double* vv = xh + 2 * N;
-  using F = SkewScratch<KPL>;
+  using F = SkewScratch<N>;
+  // With a tile of shared memory for every warp the from-scratch tiles serve as fetch buffers between recomputes: a
+  // warp requests its next projection as soon as it is done with one, and its first one of the next pass ahead of the
+  // candidate.
+  const bool staged = ntile >= nwarps;
+  double* buf = (double*)(smem + tile_off) + (size_t)warp * N * N;
+  bool ahead = false;  // the warp's first projection has been requested
+  auto G0 = [&](int qp) { return c.Yw + (size_t)qp * N * N; };
 
   for (int k = tid; k < 625; k += blockDim.x) s.mt[k] = W.mt[(size_t)w * 625 + k];
   if (tid == 0) {
@@ -467,6 +550,9 @@ __global__ void __launch_bounds__(kSkThreads, 1)
   int naccept = 0, nacc_tmp = 0, nacc_all = 0;
   for (int i0 = -d.nwarm; i0 <= d.ns && !status(c); i0++) {
     if (nacc_tmp > nfastup) {
+      fetch_wait();
+      ahead = false;
+      __syncthreads();
       checkpoint<0, 0, F>(c, nfastup, i0);
       if (status(c)) break;
       nacc_tmp = 0;
@@ -478,9 +564,14 @@ __global__ void __launch_bounds__(kSkThreads, 1)
       }
       __syncthreads();
       if (s.iflag[F_FLIP]) {
+        fetch_wait();
+        ahead = false;
+        __syncthreads();
         global_flip<0, 0, F>(c);
         if (status(c)) break;
       }
+      if (staged && !ahead && warp < d.n_qp) fetch_tile<N>(buf, G0(warp));
+      ahead = staged;
       if (tid == 0) candidate_search(c);
       __syncthreads();
       if (status(c)) break;
@@ -496,8 +587,10 @@ __global__ void __launch_bounds__(kSkThreads, 1)
       __syncthreads();
       double pre = 0.0, pim = 0.0;
       for (int qp = warp; qp < d.n_qp; qp += nwarps) {
-        const double R = warp_skew_ratio<KPL>(d, p, c.Yw + (size_t)qp * N * N, qp, s.idx, i3, i4, ra_new, rb_new,
-                                              xh, yh);
+        const double R = staged
+            ? warp_skew_ratio<N>(d, p, buf, qp, s.idx, i3, i4, ra_new, rb_new, xh, yh, true)
+            : warp_skew_ratio<N>(d, p, G0(qp), qp, s.idx, i3, i4, ra_new, rb_new, xh, yh, false);
+        if (staged) fetch_tile<N>(buf, G0(qp + nwarps < d.n_qp ? qp + nwarps : warp));
         if (lane == 0) {
           const double pfn = R * s.pf[qp];
           s.pfp[qp] = pfn;
@@ -529,9 +622,14 @@ __global__ void __launch_bounds__(kSkThreads, 1)
       }
       __syncthreads();
       if (s.iflag[F_ACCEPT]) {  // make_sample.f90:205-219
-        for (int qp = warp; qp < d.n_qp; qp += nwarps)
-          warp_skew_update<KPL>(d, p, c.Yw + (size_t)qp * N * N, qp, s.idx, i3, i4, ra_old, rb_old, ra_new, rb_new,
-                                xh, yh, vv);
+        for (int qp = warp; qp < d.n_qp; qp += nwarps) {
+          if (staged)
+            warp_skew_update<N>(d, p, buf, G0(qp), qp, s.idx, i3, i4, ra_old, rb_old, ra_new, rb_new, xh, yh, vv, true);
+          else
+            warp_skew_update<N>(d, p, G0(qp), G0(qp), qp, s.idx, i3, i4, ra_old, rb_old, ra_new, rb_new, xh,
+                                yh, vv, false);
+          if (staged) fetch_tile<N>(buf, G0(qp + nwarps < d.n_qp ? qp + nwarps : warp));
+        }
         for (int j = tid; j < d.Mr; j += blockDim.x) s.th[j] = s.thp[j];
         for (int mp = tid; mp < d.n_mp; mp += blockDim.x) s.sgn[mp] = s.sgnp[mp];
         for (int qp = tid; qp < d.n_qp; qp += blockDim.x) {
@@ -573,6 +671,7 @@ __global__ void __launch_bounds__(kSkThreads, 1)
     }
     __syncthreads();
   }
+  fetch_wait();
   for (int k = tid; k < 625; k += blockDim.x) W.mt[(size_t)w * 625 + k] = s.mt[k];
   for (int i = tid; i < N; i += blockDim.x) {
     W.x[(size_t)w * N + i] = (int8_t)s.x[i];
@@ -667,7 +766,10 @@ __device__ __forceinline__ void skew_coef(const DevDims& d, int sp, bool dn_i, b
   }
 }
 
-template <int KPL>
+// One CTA per configuration, a warp per projection: the elimination and the bonds' G y^ products are chains of
+// shared-memory loads.  Measured with N a constant, the gather of B in batches and the elimination's multipliers
+// divided once: 8.2 -> 5.5 ms for 256 configurations at 6x6 with translations.
+template <int N>
 __global__ void __launch_bounds__(kSkThreads, 1)
     estimator_skew_kernel(const __grid_constant__ DevDims d, const __grid_constant__ DevTables t,
                           const __grid_constant__ DevParams p, const int8_t* xs, int n, double* out_psi,
@@ -678,7 +780,7 @@ __global__ void __launch_bounds__(kSkThreads, 1)
   if (threadIdx.x == 0) skest_layout(d, nqw, smem, &s, &e);
   __syncthreads();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int N = d.N, Np = d.Np, ld = N + 1, NB = 4 * N;
+  constexpr int Np = N / 2, ld = N + 1, NB = 4 * N, KPL = kpl(N);
   const int cfgi = blockIdx.x;
   if (cfgi >= n) return;
   double* Orow = O ? O + (size_t)cfgi * d.Nv : nullptr;
@@ -738,13 +840,13 @@ __global__ void __launch_bounds__(kSkThreads, 1)
       const int mp = qp >> 1, sp = qp & 1;
       double* T = e.tiles + (size_t)warp * N * ld;
       int* src = e.perm + (size_t)warp * N;
-      warp_gather_skew(T, d, p, qp, s.idx);
+      warp_gather_skew<N>(T, p, qp, s.idx);
       bool sing;
-      const double pfq = warp_pfaffian<KPL>(T, N, sing);
+      const double pfq = warp_pfaffian<N>(T, sing);
       if (!sing) {
-        warp_gather_skew(T, d, p, qp, s.idx);
-        (void)warp_gj<KPL, 0, 4>(T, N, src, sing);
-        if (!sing) warp_unpermute_skew<KPL>(T, N, src);
+        warp_gather_skew<N>(T, p, qp, s.idx);
+        (void)warp_gj<KPL, N, 4>(T, N, src, sing);
+        if (!sing) warp_unpermute_skew<N>(T, src);
       }
       if (sing) bad = 1;
       const cplx cw = psi_wo_pf(d, t, s.rbm[qp], s.sgn[mp], qp);
@@ -758,9 +860,9 @@ __global__ void __launch_bounds__(kSkThreads, 1)
         const int i1 = e.ap[2 * b], i2 = e.ap[2 * b + 1];
         const int ea = s.cfg[i1], eb = s.cfg[i2];  // electron ea moves to i2, eb to i1
         const int ra = i2 + (ea >= Np ? N : 0), rb = i1 + (eb >= Np ? N : 0);
-        const double* SEa = se_row(d, p, qp, ra);
-        const double* SEb = se_row(d, p, qp, rb);
-        warp_gather_xy(d, SEa, SEb, s.idx, ea, eb, xh, yh);
+        const double* SEa = se_row<N>(p, qp, ra);
+        const double* SEb = se_row<N>(p, qp, rb);
+        warp_gather_xy<N>(SEa, SEb, s.idx, ea, eb, xh, yh);
         const double ya = -SEa[rb];
         // (G y^)_i for this lane's rows
         double xgy = 0.0;
@@ -910,9 +1012,11 @@ int max_smem_optin() {
   return maxsm;
 }
 
-int skew_sampler_tiles(const DevDims& d, int maxsm) {
-  for (int q = kSkWarps; q >= 1; q--)
-    if ((long long)skew_sampler_smem(d, q, nullptr, nullptr) <= maxsm) return q;
+// From-scratch tiles of the sampler's block (0: the shape does not fit) and its warps
+int skew_sampler_tiles(const DevDims& d, int maxsm, int& nwarps) {
+  for (nwarps = kSmpThreads / 32; nwarps >= kSkWarps; nwarps /= 2)
+    for (int q = nwarps; q >= 1; q--)
+      if ((long long)skew_sampler_smem(d, nwarps, q, nullptr, nullptr) <= maxsm) return q;
   return 0;
 }
 
@@ -930,7 +1034,8 @@ int rbmpp_skew_max_n() { return 128; }
 // 0 when the skew sampler and estimator fit one block's shared memory at this shape, else the bytes one of them
 // needs at its smallest.
 size_t rbmpp_skew_smem_shortfall(const DevDims& d, int maxsm) {
-  if (skew_sampler_tiles(d, maxsm) < 1) return skew_sampler_smem(d, 1, nullptr, nullptr);
+  int nwarps = 0;
+  if (skew_sampler_tiles(d, maxsm, nwarps) < 1) return skew_sampler_smem(d, kSkWarps, 1, nullptr, nullptr);
   if (skew_est_tiles(d, maxsm) < 1) return skest_layout(d, 1, nullptr, nullptr, nullptr);
   return 0;
 }
@@ -947,23 +1052,27 @@ cudaError_t rbmpp_build_se(const DevDims& d, const int* wmap, const int* orb, co
 
 cudaError_t rbmpp_launch_sampler_skew(const DevDims& d, const DevTables& t, const DevParams& p, const DevWalkers& W,
                                       int first, cudaStream_t st) {
-  const int ntile = skew_sampler_tiles(d, max_smem_optin());
-  if (ntile < 1 || d.N > rbmpp_skew_max_n()) return cudaErrorInvalidValue;
-  const size_t smem = skew_sampler_smem(d, ntile, nullptr, nullptr);
-#define LAUNCH_SK(K)                                                                                            \
-  do {                                                                                                          \
-    cudaError_t e = cudaFuncSetAttribute(sampler_skew_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,   \
-                                         (int)smem);                                                            \
-    if (e != cudaSuccess) return e;                                                                             \
-    rbmpp_note_launch();                                                                                        \
-    sampler_skew_kernel<K><<<d.nw, kSkThreads, smem, st>>>(d, t, p, W, first, ntile);                           \
-    return cudaGetLastError();                                                                                  \
+  int nwarps = 0;
+  const int ntile = skew_sampler_tiles(d, max_smem_optin(), nwarps);
+  if (ntile < 1) return cudaErrorInvalidValue;
+  const size_t smem = skew_sampler_smem(d, nwarps, ntile, nullptr, nullptr);
+#define LAUNCH_SK(K)                                                                                                \
+  do {                                                                                                              \
+    cudaError_t e = cudaFuncSetAttribute(sampler_skew_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,       \
+                                         (int)smem);                                                                \
+    if (e != cudaSuccess) return e;                                                                                 \
+    rbmpp_note_launch();                                                                                            \
+    sampler_skew_kernel<K><<<d.nw, 32 * nwarps, smem, st>>>(d, t, p, W, first, ntile);                              \
+    return cudaGetLastError();                                                                                      \
   } while (0)
-  const int kpl = (d.N + 31) / 32;
-  if (kpl <= 1) LAUNCH_SK(1);
-  if (kpl <= 2) LAUNCH_SK(2);
-  if (kpl <= 3) LAUNCH_SK(3);
-  LAUNCH_SK(4);
+  switch (d.N) {
+    case 4: LAUNCH_SK(4);
+    case 16: LAUNCH_SK(16);
+    case 36: LAUNCH_SK(36);
+    case 64: LAUNCH_SK(64);
+    case 100: LAUNCH_SK(100);
+    default: return cudaErrorInvalidValue;
+  }
 #undef LAUNCH_SK
 }
 
@@ -972,7 +1081,7 @@ cudaError_t rbmpp_launch_estimator_skew(const DevDims& d, const DevTables& t, co
                                         int* out_status, int reweight, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
   const int nqw = skew_est_tiles(d, max_smem_optin());
-  if (nqw < 1 || d.N > rbmpp_skew_max_n()) return cudaErrorInvalidValue;
+  if (nqw < 1) return cudaErrorInvalidValue;
   const size_t smem = skest_layout(d, nqw, nullptr, nullptr, nullptr);
 #define LAUNCH_SE(K)                                                                                             \
   do {                                                                                                           \
@@ -984,10 +1093,13 @@ cudaError_t rbmpp_launch_estimator_skew(const DevDims& d, const DevTables& t, co
                                                           out_status, reweight, nqw);                            \
     return cudaGetLastError();                                                                                   \
   } while (0)
-  const int kpl = (d.N + 31) / 32;
-  if (kpl <= 1) LAUNCH_SE(1);
-  if (kpl <= 2) LAUNCH_SE(2);
-  if (kpl <= 3) LAUNCH_SE(3);
-  LAUNCH_SE(4);
+  switch (d.N) {
+    case 4: LAUNCH_SE(4);
+    case 16: LAUNCH_SE(16);
+    case 36: LAUNCH_SE(36);
+    case 64: LAUNCH_SE(64);
+    case 100: LAUNCH_SE(100);
+    default: return cudaErrorInvalidValue;
+  }
 #undef LAUNCH_SE
 }
