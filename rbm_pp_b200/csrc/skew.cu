@@ -17,8 +17,8 @@
 // (a skew L T L^T; restated from M. Wimmer, ACM TOMS 38(4) 2012, the role of dskpfa('U', 'P')), the inverse by
 // warp Gauss-Jordan, skew-symmetrised as matrix.f90:96-105 does, with its skew check.
 //
-// Kernels: the direct Metropolis sampler (one CTA per walker, one warp per projection at a time, G streamed
-// from HBM), the estimator (one CTA per configuration; local energy over the antiparallel J1/J2 bonds,
+// Kernels: the direct Metropolis sampler (one CTA or cluster per walker, a warp per projection at a time, G streamed
+// from L2 or HBM), the estimator (one CTA per configuration; local energy over the antiparallel J1/J2 bonds,
 // dPf/df_k over the four spin blocks of slater.f90:140-167) and the Slater-element table.
 #include "sampler_common.cuh"
 
@@ -38,6 +38,49 @@ constexpr int kSmpThreads = 512;
 constexpr int kpl(int N) { return (N + 31) / 32; }
 constexpr int rows_read(int N) { return N == 36 ? 12 : N == 100 ? 10 : 16; }
 constexpr int rows_update(int N) { return N == 36 ? 6 : N == 100 ? 5 : 8; }
+
+// A walker's block, or its cluster of blocks: every block carries the whole walker state (one random sequence, the same
+// decisions from the same numbers) and owns every size-th projection, so a G is touched by one block only.  What the
+// blocks exchange: the Pfaffians and drift of a from-scratch pass, and every proposal's partial sums.
+constexpr int kMaxCluster = 8;
+struct Team {
+  int rank, size;
+  double* slots;  // shared, with size > 1: [2][size * warps][2] partial sums by parity of the proposal, then [size][2]
+  __device__ __forceinline__ int nwarps() const { return blockDim.x >> 5; }
+  // the i-th projection that this block owns
+  __device__ __forceinline__ int own(int i) const { return i * size + rank; }
+  // barrier of all threads of the walker, with the memory order of __syncthreads over the cluster
+  __device__ __forceinline__ void sync() const {
+    if (size == 1) {
+      __syncthreads();
+    } else {
+      asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+      asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    }
+  }
+  // *p = v in the shared memory of every block of the walker (visible after the next sync)
+  __device__ __forceinline__ void put(double* p, double v) const {
+    *p = v;
+    for (int r = 0; r < size; r++)
+      if (r != rank) {
+        uint32_t a;
+        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(r));
+        asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+      }
+  }
+};
+// TEAM: the kernel was launched in clusters (one block: rank and size are constants)
+template <bool TEAM>
+__device__ __forceinline__ Team team(double* slots) {
+  Team m{0, 1, slots};
+  if (TEAM) {
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(m.rank));
+    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(m.size));
+  }
+  return m;
+}
+// doubles of Team::slots: they lie in the per-warp vectors of the block form, which the skew form does not use
+__host__ __device__ __forceinline__ int team_slots(int nwarps, int size) { return 4 * size * nwarps + 2 * size; }
 
 __device__ __forceinline__ int rho_of(const int* idx, int e, int Np, int N) { return idx[e] + (e >= Np ? N : 0); }
 
@@ -202,11 +245,13 @@ __device__ void warp_unpermute_skew(double* T, const int* perm) {
 // calculate_MAll for the skew form (policy of the walker routines of sampler_common.cuh): one warp per
 // projection on its own shared-memory tile; writes G (when write_y) and pf_out; with diff, the drift measure
 // of make_sample.f90:106-113 against the stored G.
-template <int N>
+template <int N, bool TEAM>
 struct SkewScratch {
   static __device__ void run(const SCtx& c, const int* idx, double* pf_out, bool write_y, bool diff) {
     const DevDims& d = c.d;
     const WS& s = c.s;
+    const Team m = team<TEAM>(s.wv);
+    if (m.size > 1) m.sync();  // every block is done with pf_out and the slots
     constexpr int ld = N + 1, KPL = kpl(N);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     double wratio = -1.0;
@@ -214,7 +259,7 @@ struct SkewScratch {
     if (warp < c.par_ntile) {
       double* T = c.par_tiles + (size_t)warp * N * ld;
       int* perm = (int*)(s.wS + (size_t)warp * d.Np);
-      for (int qp = warp; qp < d.n_qp && !bad; qp += c.par_ntile) {
+      for (int i = warp, qp; (qp = m.own(i)) < d.n_qp && !bad; i += c.par_ntile) {
         warp_gather_skew<N>(T, c.p, qp, idx);
         bool sing;
         const double pfq = warp_pfaffian<N>(T, sing);
@@ -244,7 +289,7 @@ struct SkewScratch {
         msym = warp_max(msym);
         if (msym > 2.0e-3 * mraw) bad = 2;
         if (diff) wratio = fmax(wratio, md / mx);
-        if (lane == 0) pf_out[qp] = pfq;
+        if (lane == 0) m.put(pf_out + qp, pfq);
         __syncwarp();
       }
     }
@@ -260,10 +305,30 @@ struct SkewScratch {
         di = fmax(di, s.red[w]);
         if (s.red[32 + w] != 0.0 && !b) b = (int)s.red[32 + w];
       }
-      if (b) status(c) = b == 1 ? ST_SINGULAR : ST_SKEW;
-      s.dsc[D_DIFFINV] = di;
+      if (m.size > 1) {
+        double* part = m.slots + 4 * m.size * m.nwarps();
+        m.put(part + 2 * m.rank, di);
+        m.put(part + 2 * m.rank + 1, (double)b);
+      } else {
+        if (b) status(c) = b == 1 ? ST_SINGULAR : ST_SKEW;
+        s.dsc[D_DIFFINV] = di;
+      }
     }
-    __syncthreads();
+    m.sync();
+    if (m.size > 1) {
+      if (threadIdx.x == 0) {
+        const double* part = m.slots + 4 * m.size * m.nwarps();
+        double di = -1.0;
+        int b = 0;
+        for (int r = 0; r < m.size; r++) {
+          di = fmax(di, part[2 * r]);
+          if (part[2 * r + 1] != 0.0 && !b) b = (int)part[2 * r + 1];
+        }
+        if (b) status(c) = b == 1 ? ST_SINGULAR : ST_SKEW;
+        s.dsc[D_DIFFINV] = di;
+      }
+      __syncthreads();
+    }
   }
 };
 
@@ -493,16 +558,18 @@ __host__ __device__ size_t skew_sampler_smem(const DevDims& d, int nwarps, int n
 // Bounded by instructions on the SMs that have a walker: with the walker's G in L2 (72 projections of 10 KB at 6x6) a
 // proposal is an x^ . G y^ product per projection, 2,800 warp instructions each before N was a constant.  Measured,
 // make_sample of 64 walkers, 6x6 with translations, 35 sweeps: 104 -> 65 ms with 16 warps, row batches and staged
-// fetches (8 warps, two rows in flight, straight from L2), -> 49 ms with N a constant.
-template <int N>
+// fetches (8 warps, two rows in flight, straight from L2), -> 49 ms with N a constant, -> 33 ms with two blocks per
+// walker.
+template <int N, bool TEAM>
 __global__ void __launch_bounds__(kSmpThreads, 1)
     sampler_skew_kernel(const __grid_constant__ DevDims d, const __grid_constant__ DevTables t,
                         const __grid_constant__ DevParams p, const __grid_constant__ DevWalkers W, int first,
                         int ntile) {
   extern __shared__ __align__(16) char smem[];
   __shared__ WS ws;
-  const int w = blockIdx.x;
-  if (w >= d.nw) return;
+  const Team m0 = team<TEAM>(nullptr);
+  const int w = blockIdx.x / m0.size;
+  if (w >= d.nw) return;  // all blocks of a walker
   size_t vec_off = 0, tile_off = 0;
   skew_sampler_smem(d, blockDim.x >> 5, ntile, &vec_off, &tile_off);
   if (threadIdx.x == 0) ws_layout(d, blockDim.x >> 5, smem, &ws, false);
@@ -510,11 +577,12 @@ __global__ void __launch_bounds__(kSmpThreads, 1)
   constexpr int Np = N / 2;
   const SCtx c{d, t, p, W, w, ws, W.Y + (size_t)w * d.n_qp * N * N, (double*)(smem + tile_off), ntile};
   const WS& s = ws;
+  const Team m{m0.rank, m0.size, s.wv};
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nwarps = blockDim.x >> 5;
   double* xh = (double*)(smem + vec_off) + (size_t)warp * 6 * N;
   double* yh = xh + N;
   double* vv = xh + 2 * N;
-  using F = SkewScratch<N>;
+  using F = SkewScratch<N, TEAM>;
   // With a tile of shared memory for every warp the from-scratch tiles serve as fetch buffers between recomputes: a
   // warp requests its next projection as soon as it is done with one, and its first one of the next pass ahead of the
   // candidate.
@@ -522,6 +590,8 @@ __global__ void __launch_bounds__(kSmpThreads, 1)
   double* buf = (double*)(smem + tile_off) + (size_t)warp * N * N;
   bool ahead = false;  // the warp's first projection has been requested
   auto G0 = [&](int qp) { return c.Yw + (size_t)qp * N * N; };
+  const int qp0 = m.own(warp), qstep = m.size * nwarps;  // the warp's projections
+  int parity = 0;
 
   for (int k = tid; k < 625; k += blockDim.x) s.mt[k] = W.mt[(size_t)w * 625 + k];
   if (tid == 0) {
@@ -552,7 +622,11 @@ __global__ void __launch_bounds__(kSmpThreads, 1)
     if (nacc_tmp > nfastup) {
       fetch_wait();
       ahead = false;
-      __syncthreads();
+      if (m.size > 1) {  // the drift measure takes the Pfaffians of all projections
+        m.sync();
+        for (int i = tid; m.own(i) < d.n_qp; i += blockDim.x) m.put(s.pf + m.own(i), s.pf[m.own(i)]);
+      }
+      m.sync();
       checkpoint<0, 0, F>(c, nfastup, i0);
       if (status(c)) break;
       nacc_tmp = 0;
@@ -570,7 +644,7 @@ __global__ void __launch_bounds__(kSmpThreads, 1)
         global_flip<0, 0, F>(c);
         if (status(c)) break;
       }
-      if (staged && !ahead && warp < d.n_qp) fetch_tile<N>(buf, G0(warp));
+      if (staged && !ahead && qp0 < d.n_qp) fetch_tile<N>(buf, G0(qp0));
       ahead = staged;
       if (tid == 0) candidate_search(c);
       __syncthreads();
@@ -586,11 +660,11 @@ __global__ void __launch_bounds__(kSmpThreads, 1)
       cta_rbm_factors(d, s.thp, s.rbm);
       __syncthreads();
       double pre = 0.0, pim = 0.0;
-      for (int qp = warp; qp < d.n_qp; qp += nwarps) {
+      for (int qp = qp0; qp < d.n_qp; qp += qstep) {
         const double R = staged
             ? warp_skew_ratio<N>(d, p, buf, qp, s.idx, i3, i4, ra_new, rb_new, xh, yh, true)
             : warp_skew_ratio<N>(d, p, G0(qp), qp, s.idx, i3, i4, ra_new, rb_new, xh, yh, false);
-        if (staged) fetch_tile<N>(buf, G0(qp + nwarps < d.n_qp ? qp + nwarps : warp));
+        if (staged) fetch_tile<N>(buf, G0(qp + qstep < d.n_qp ? qp + qstep : qp0));
         if (lane == 0) {
           const double pfn = R * s.pf[qp];
           s.pfp[qp] = pfn;
@@ -601,16 +675,22 @@ __global__ void __launch_bounds__(kSmpThreads, 1)
           pim += cw.im * pfn;
         }
       }
+      // partial sums of all warps of the walker; a block may be one proposal ahead of another, so two sets of slots
+      double* part = m.size > 1 ? m.slots + 2 * parity * qstep : s.red;
+      parity ^= 1;
       if (lane == 0) {
-        s.red[warp] = pre;
-        s.red[32 + warp] = pim;
+        m.put(part + m.rank * nwarps + warp, pre);
+        m.put(part + (m.size > 1 ? qstep : 32) + m.rank * nwarps + warp, pim);
       }
-      __syncthreads();
+      m.sync();
       if (tid == 0) {
         double re = 0.0, im = 0.0;
-        for (int k = 0; k < nwarps; k++) {
-          re += s.red[k];
-          im += s.red[32 + k];
+        const double* pi = part + (m.size > 1 ? qstep : 32);
+        const int nsum = m.size > 1 ? qstep : min(nwarps, d.n_qp);  // warps with a projection
+#pragma unroll 4
+        for (int k = 0; k < nsum; k++) {
+          re += part[k];
+          im += pi[k];
         }
         s.dsc[D_PSIPR] = re;
         s.dsc[D_PSIPI] = im;
@@ -622,17 +702,17 @@ __global__ void __launch_bounds__(kSmpThreads, 1)
       }
       __syncthreads();
       if (s.iflag[F_ACCEPT]) {  // make_sample.f90:205-219
-        for (int qp = warp; qp < d.n_qp; qp += nwarps) {
+        for (int qp = qp0; qp < d.n_qp; qp += qstep) {
           if (staged)
             warp_skew_update<N>(d, p, buf, G0(qp), qp, s.idx, i3, i4, ra_old, rb_old, ra_new, rb_new, xh, yh, vv, true);
           else
             warp_skew_update<N>(d, p, G0(qp), G0(qp), qp, s.idx, i3, i4, ra_old, rb_old, ra_new, rb_new, xh,
                                 yh, vv, false);
-          if (staged) fetch_tile<N>(buf, G0(qp + nwarps < d.n_qp ? qp + nwarps : warp));
+          if (staged) fetch_tile<N>(buf, G0(qp + qstep < d.n_qp ? qp + qstep : qp0));
         }
         for (int j = tid; j < d.Mr; j += blockDim.x) s.th[j] = s.thp[j];
         for (int mp = tid; mp < d.n_mp; mp += blockDim.x) s.sgn[mp] = s.sgnp[mp];
-        for (int qp = tid; qp < d.n_qp; qp += blockDim.x) {
+        for (int i = tid, qp; (qp = m.own(i)) < d.n_qp; i += blockDim.x) {
           s.pf[qp] = s.pfp[qp];
           s.psi[2 * qp] = s.psip[2 * qp];
           s.psi[2 * qp + 1] = s.psip[2 * qp + 1];
@@ -657,14 +737,15 @@ __global__ void __launch_bounds__(kSmpThreads, 1)
     if (status(c)) break;
     if (i0 > 0) {  // make_sample.f90:228-232
       const size_t sidx = (size_t)w * d.ns + (i0 - 1);
-      for (int i = tid; i < N; i += blockDim.x) W.xs[sidx * N + i] = (int8_t)s.x[i];
-      for (int qp = tid; qp < d.n_qp; qp += blockDim.x) W.pfs[sidx * d.n_qp + qp] = s.pf[qp];
+      if (m.rank == 0)
+        for (int i = tid; i < N; i += blockDim.x) W.xs[sidx * N + i] = (int8_t)s.x[i];
+      for (int i = tid, qp; (qp = m.own(i)) < d.n_qp; i += blockDim.x) W.pfs[sidx * d.n_qp + qp] = s.pf[qp];
       double* ps = W.psis + sidx * (size_t)(d.n_qp + 1) * 2;
-      for (int k = tid; k < d.n_qp; k += blockDim.x) {
+      for (int i = tid, k; (k = m.own(i)) < d.n_qp; i += blockDim.x) {
         ps[2 * (k + 1)] = s.psi[2 * k];
         ps[2 * (k + 1) + 1] = s.psi[2 * k + 1];
       }
-      if (tid == 0) {
+      if (tid == 0 && m.rank == 0) {
         ps[0] = s.dsc[D_PSI0R];
         ps[1] = s.dsc[D_PSI0I];
       }
@@ -672,6 +753,8 @@ __global__ void __launch_bounds__(kSmpThreads, 1)
     __syncthreads();
   }
   fetch_wait();
+  if (m.size > 1) m.sync();  // no block leaves while another may still write to it
+  if (m.rank) return;
   for (int k = tid; k < 625; k += blockDim.x) W.mt[(size_t)w * 625 + k] = s.mt[k];
   for (int i = tid; i < N; i += blockDim.x) {
     W.x[(size_t)w * N + i] = (int8_t)s.x[i];
@@ -1026,6 +1109,49 @@ int skew_est_tiles(const DevDims& d, int maxsm) {
   return 0;
 }
 
+// Blocks per walker: the largest power of two whose blocks all have a projection, if the device holds every walker's
+// cluster at the same time (a second wave of walkers costs more than the split gives).  Measured, 35 sweeps with
+// translations, one block, two, and the choice of this rule: 6x6, 74 walkers 44 / 29.7 / 29.7 ms (two), 32 walkers 44 /
+// 29.7 / 21.5 (four); 8x8, 30 walkers 203 (two) / 125 (four), 8 walkers 162 (two) / 54 (eight).  With only two
+// projections (no translations) a walker keeps one block: 9.1 ms at 6x6, 10.5 with the cluster's barriers.
+cudaError_t launch_skew_sampler(const void* kernel, const void* team_kernel, DevDims d, DevTables t, DevParams p,
+                                DevWalkers W, int first, int ntile, int nwarps, size_t smem, cudaStream_t st) {
+  cudaError_t e;
+  for (const void* k : {kernel, team_kernel})
+    if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess) return e;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.blockDim = dim3(32 * nwarps);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  int dev = 0, nsm = 0, size = kMaxCluster;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  for (; size > 1; size /= 2) {
+    if ((size - 1) * nwarps >= d.n_qp || team_slots(nwarps, size) > 2 * nwarps * d.Np || d.nw * size > nsm)
+      continue;
+    at.val.clusterDim.x = size;
+    cfg.gridDim = dim3(d.nw * size);
+    int held = 0;
+    if (cudaOccupancyMaxActiveClusters(&held, team_kernel, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      continue;
+    }
+    if (held >= d.nw) break;
+  }
+  at.val.clusterDim.x = size;
+  cfg.gridDim = dim3(d.nw * size);
+  if (size == 1) cfg.numAttrs = 0;
+  void* args[] = {&d, &t, &p, &W, &first, &ntile};
+  rbmpp_note_launch();
+  e = cudaLaunchKernelExC(&cfg, size > 1 ? team_kernel : kernel, args);
+  return e != cudaSuccess ? e : cudaGetLastError();
+}
+
 }  // namespace
 
 // Largest N the skew kernels take (lanes hold N / 32 columns each).
@@ -1056,21 +1182,15 @@ cudaError_t rbmpp_launch_sampler_skew(const DevDims& d, const DevTables& t, cons
   const int ntile = skew_sampler_tiles(d, max_smem_optin(), nwarps);
   if (ntile < 1) return cudaErrorInvalidValue;
   const size_t smem = skew_sampler_smem(d, nwarps, ntile, nullptr, nullptr);
-#define LAUNCH_SK(K)                                                                                                \
-  do {                                                                                                              \
-    cudaError_t e = cudaFuncSetAttribute(sampler_skew_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,       \
-                                         (int)smem);                                                                \
-    if (e != cudaSuccess) return e;                                                                                 \
-    rbmpp_note_launch();                                                                                            \
-    sampler_skew_kernel<K><<<d.nw, 32 * nwarps, smem, st>>>(d, t, p, W, first, ntile);                              \
-    return cudaGetLastError();                                                                                      \
-  } while (0)
+#define LAUNCH_SK(K, T)                                                                                              \
+  return launch_skew_sampler((const void*)sampler_skew_kernel<K, false>, (const void*)sampler_skew_kernel<K, T>, d, \
+                             t, p, W, first, ntile, nwarps, smem, st)
   switch (d.N) {
-    case 4: LAUNCH_SK(4);
-    case 16: LAUNCH_SK(16);
-    case 36: LAUNCH_SK(36);
-    case 64: LAUNCH_SK(64);
-    case 100: LAUNCH_SK(100);
+    case 4: LAUNCH_SK(4, false);  // at most 8 projections: one block
+    case 16: LAUNCH_SK(16, true);
+    case 36: LAUNCH_SK(36, true);
+    case 64: LAUNCH_SK(64, true);
+    case 100: LAUNCH_SK(100, true);
     default: return cudaErrorInvalidValue;
   }
 #undef LAUNCH_SK

@@ -1,7 +1,7 @@
 """The skew form's kernels over the lattice sizes and numbers of walkers (skew.cu): every even square lattice is an
-instance of its own; small lattices keep a fetch buffer per warp, large ones read the inverse matrices in place.
-Chains are compared with the oracle's decision by decision, amplitudes, local energies and derivatives of given
-configurations with its values."""
+instance of its own; few walkers have a cluster of blocks each, many one block; small lattices keep a fetch buffer per
+warp, large ones read the inverse matrices in place.  Chains are compared with the oracle's decision by decision,
+amplitudes, local energies and derivatives of given configurations with its values."""
 import numpy as np
 import pytest
 
@@ -14,8 +14,9 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("L,trans,nw,ns", [
     (4, True, 3, 8),
     (4, False, 160, 1),  # more walkers than SMs
-    (6, True, 2, 2),
-    (6, True, 40, 1),
+    (6, True, 2, 2),     # four blocks per walker
+    (6, True, 40, 1),    # two
+    (8, True, 1, 1),     # eight
     (8, False, 4, 1),
     (10, False, 2, 1),
 ])
