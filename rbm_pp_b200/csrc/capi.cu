@@ -34,7 +34,7 @@ size_t rbmpp_estimator_smem_any(const DevDims&, int);
 cudaError_t rbmpp_launch_advance_rng(uint32_t*, const int*, int, int, int, cudaStream_t);
 cudaError_t rbmpp_syrk_ot_o(int, int, const double*, double*, cudaStream_t);
 cudaError_t rbmpp_symmetrize(int, double*, cudaStream_t);
-cudaError_t rbmpp_potrf_upper(int, double*, double*, int*, cudaStream_t);
+cudaError_t rbmpp_potrf_upper(int, double*, double*, int*, cudaStream_t, cudaStream_t, cudaEvent_t, cudaEvent_t);
 cudaError_t rbmpp_potrs_upper(int, const double*, const double*, double*, double*, unsigned*, cudaStream_t);
 int rbmpp_gram_parts();
 size_t rbmpp_chol_work(int);
@@ -180,6 +180,8 @@ struct rbmpp_ctx {
   double wf_av_list[10] = {0};
   size_t bytes = 0;
   cudaEvent_t ev[12] = {};
+  cudaStream_t st_side = nullptr;  // the Cholesky's diagonal blocks, beside its trailing products on st
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   double stats[10] = {0};
   int stream_stages = 0;  // > 0: TMA-streamed sampler with this many stages
   bool sampler_auto = true;  // RBMPP_SAMPLER did not choose the direct sampler
@@ -601,6 +603,9 @@ int rbmpp_destroy(rbmpp_ctx* c) {
   if (c->h_sc) cudaFreeHost(c->h_sc);
   for (auto& e : c->ev)
     if (e) cudaEventDestroy(e);
+  if (c->ev_fork) cudaEventDestroy(c->ev_fork);
+  if (c->ev_join) cudaEventDestroy(c->ev_join);
+  if (c->st_side) cudaStreamDestroy(c->st_side);
   if (c->st) cudaStreamDestroy(c->st);
   delete c;
   return 0;
@@ -1191,11 +1196,18 @@ int rbmpp_sr_step(rbmpp_ctx* c, const rbmpp_sr_in* in, rbmpp_sr_out* out, double
     }
     CK(cudaMemcpyAsync(c->d_Sb, c->d_S, s_bytes, cudaMemcpyDeviceToDevice, c->st));
   }
+  if (!c->st_side) {  // kept for the next steps
+    int prio_low = 0, prio_high = 0;
+    CK(cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high));
+    if (!c->ev_fork) CK(cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
+    if (!c->ev_join) CK(cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming));
+    CK(cudaStreamCreateWithPriority(&c->st_side, cudaStreamNonBlocking, prio_high));
+  }
   int info = 0, attempts = 0;
   double tau = 0.0;
   for (int attempt = 0;; attempt++) {
     attempts = attempt + 1;
-    CK(rbmpp_potrf_upper(Nv, c->d_S, c->d_dinv, c->d_info, c->st));
+    CK(rbmpp_potrf_upper(Nv, c->d_S, c->d_dinv, c->d_info, c->st, c->st_side, c->ev_fork, c->ev_join));
     CK(cudaMemcpyAsync(&info, c->d_info, sizeof(int), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
     if (info == 0 || in->precision != RBMPP_SR_SPLIT_BF16 || in->refine_steps <= 0 || attempt == 12) break;

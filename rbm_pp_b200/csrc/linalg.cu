@@ -16,7 +16,8 @@ namespace {
 // Bound by the FP64 pipe (37 TFLOP/s by mma.m8n8k4.f64, measured; 33 by FMA).  At BM = 128 eight warps hold 64 x 32
 // accumulators each (32 pieces of 8 x 8), so a step of four k costs twelve shared loads for 32 products; operands come
 // by cp.async into kStages buffers.  Both operands are kept as [k][i] (row length 4 mod 16) or, with KCONTIG, [i][k]
-// (likewise), which puts an 8 x 4 fragment on distinct banks either way.  VEC = 2: 16-byte copies, for a base and a
+// (likewise), which puts an 8 x 4 fragment on distinct banks either way.  Columns j < jmin stay as they are (the
+// Cholesky's next diagonal block, which sr_solve.cu updates itself).  VEC = 2: 16-byte copies, for a base and a
 // stride of whole 16-byte words; an odd stride takes 8-byte ones.
 // Measured against the form before (FMA, 8 x 8 results a thread, loads one step ahead): the S build of 8192 samples x
 // 4226 parameters 13.2 -> 5.8 ms, factorisation and solve of 10404 parameters 56.3 -> 34.3 ms.
@@ -67,7 +68,7 @@ __device__ __forceinline__ void load_operand(double* dst, const double* __restri
 template <int BM, bool KCONTIG, bool ACC, int VEC>
 __global__ void __launch_bounds__(256, BM > 64 ? 1 : 2) gemm_atb_upper(int n, int K, const double* __restrict__ A, long long sk,
                                                          long long si, double alpha, double* __restrict__ C,
-                                                         long long ldc, int row0) {
+                                                         long long ldc, int row0, int jmin) {
   // upper-tile index -> (ti, tj) with ti <= tj
   const int nt = (n - row0 + BM - 1) / BM;
   int t = blockIdx.x, ti = 0;
@@ -77,6 +78,7 @@ __global__ void __launch_bounds__(256, BM > 64 ? 1 : 2) gemm_atb_upper(int n, in
   }
   const int tj = ti + t;
   const int i0 = row0 + ti * BM, j0 = row0 + tj * BM;
+  if (j0 + BM <= jmin) return;
   extern __shared__ __align__(16) double sm[];
   constexpr int TD = kTileDoubles<BM, KCONTIG>, kLdI = BM + 4, PI = BM / 16, PJ = BM / 32;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, c = lane & 3;
@@ -127,7 +129,7 @@ __global__ void __launch_bounds__(256, BM > 64 ? 1 : 2) gemm_atb_upper(int n, in
 #pragma unroll
     for (int e = 0; e < 2; e++) {
       const int j = j0 + wj + 8 * b + 2 * c + e;
-      if (j >= n) continue;
+      if (j >= n || j < jmin) continue;
       double* col = C + ldc * j;
       double old[PI];
       if (ACC) {
@@ -147,7 +149,7 @@ __global__ void __launch_bounds__(256, BM > 64 ? 1 : 2) gemm_atb_upper(int n, in
 
 template <int BM, bool KCONTIG, bool ACC>
 cudaError_t launch_gemm_bm(int n, int K, const double* A, long long sk, long long si, double alpha, double* C,
-                           long long ldc, int row0, cudaStream_t st) {
+                           long long ldc, int row0, int jmin, cudaStream_t st) {
   const int nt = (n - row0 + BM - 1) / BM;
   const long long stride = KCONTIG ? si : sk;
   const bool vec = stride % 2 == 0 && (uintptr_t)A % 16 == 0 && row0 % 2 == 0;
@@ -155,7 +157,7 @@ cudaError_t launch_gemm_bm(int n, int K, const double* A, long long sk, long lon
   cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem<BM, KCONTIG>);
   if (e != cudaSuccess) return e;
   rbmpp_note_launch();
-  f<<<nt * (nt + 1) / 2, 256, kGemmSmem<BM, KCONTIG>, st>>>(n, K, A, sk, si, alpha, C, ldc, row0);
+  f<<<nt * (nt + 1) / 2, 256, kGemmSmem<BM, KCONTIG>, st>>>(n, K, A, sk, si, alpha, C, ldc, row0, jmin);
   return cudaGetLastError();
 }
 
@@ -165,7 +167,7 @@ cudaError_t launch_gemm_bm(int n, int K, const double* A, long long sk, long lon
 // or a matrix of few tiles is what the smaller sizes are for.
 template <bool KCONTIG, bool ACC>
 cudaError_t launch_gemm_atb_upper(int n, int K, const double* A, long long sk, long long si, double alpha, double* C,
-                                  long long ldc, int row0, cudaStream_t st) {
+                                  long long ldc, int row0, int jmin, cudaStream_t st) {
   int dev = 0, nsm = 1;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
@@ -175,9 +177,9 @@ cudaError_t launch_gemm_atb_upper(int n, int K, const double* A, long long sk, l
     return (double)((tiles + slots - 1) / slots);
   };
   const double t128 = waves(128, nsm), t96 = 0.6 * waves(96, nsm), t64 = 0.6 * waves(64, 2 * nsm);
-  if (t128 <= t96 && t128 <= t64) return launch_gemm_bm<128, KCONTIG, ACC>(n, K, A, sk, si, alpha, C, ldc, row0, st);
-  if (t96 <= t64) return launch_gemm_bm<96, KCONTIG, ACC>(n, K, A, sk, si, alpha, C, ldc, row0, st);
-  return launch_gemm_bm<64, KCONTIG, ACC>(n, K, A, sk, si, alpha, C, ldc, row0, st);
+  if (t128 <= t96 && t128 <= t64) return launch_gemm_bm<128, KCONTIG, ACC>(n, K, A, sk, si, alpha, C, ldc, row0, jmin, st);
+  if (t96 <= t64) return launch_gemm_bm<96, KCONTIG, ACC>(n, K, A, sk, si, alpha, C, ldc, row0, jmin, st);
+  return launch_gemm_bm<64, KCONTIG, ACC>(n, K, A, sk, si, alpha, C, ldc, row0, jmin, st);
 }
 
 // mirror the upper triangle into the lower one
@@ -361,7 +363,7 @@ __global__ void sample_scalars_kernel(int ns, const double* psi, int psi_stride,
 // host wrappers
 // ------------------------------------------------------------------------------------------------
 cudaError_t rbmpp_syrk_ot_o(int nv, int ns, const double* O, double* S, cudaStream_t st) {
-  cudaError_t e = launch_gemm_atb_upper<false, false>(nv, ns, O, nv, 1, 1.0, S, nv, 0, st);
+  cudaError_t e = launch_gemm_atb_upper<false, false>(nv, ns, O, nv, 1, 1.0, S, nv, 0, 0, st);
   if (e) return e;
   dim3 g((nv + 31) / 32, (nv + 31) / 32);
   rbmpp_note_launch();
@@ -373,7 +375,7 @@ cudaError_t rbmpp_syrk_ot_o(int nv, int ns, const double* O, double* S, cudaStre
 cudaError_t rbmpp_gemm_atb_upper(int n, int K, const double* A, long long sk, long long si, double* C, long long ldc,
                                  cudaStream_t st) {
   if (si != 1) return cudaErrorInvalidValue;
-  return launch_gemm_atb_upper<false, false>(n, K, A, sk, 1, 1.0, C, ldc, 0, st);
+  return launch_gemm_atb_upper<false, false>(n, K, A, sk, 1, 1.0, C, ldc, 0, 0, st);
 }
 
 cudaError_t rbmpp_symmetrize(int n, double* S, cudaStream_t st) {
@@ -386,10 +388,10 @@ cudaError_t rbmpp_symmetrize(int n, double* S, cudaStream_t st) {
 // C(i, j) += alpha * sum_k A(k, i) A(k, j) on the upper triangle of rows and columns >= row0 (the trailing
 // update of the blocked Cholesky in sr_solve.cu; K = its panel width, A(k, i) contiguous in k)
 cudaError_t rbmpp_gemm_atb_upper_acc(int n, int K, const double* A, long long sk, long long si, double alpha,
-                                     double* C, long long ldc, int row0, cudaStream_t st) {
-  if (n - row0 <= 0) return cudaSuccess;
+                                     double* C, long long ldc, int row0, int jmin, cudaStream_t st) {
+  if (n - row0 <= 0 || n <= jmin) return cudaSuccess;
   if (sk != 1) return cudaErrorInvalidValue;
-  return launch_gemm_atb_upper<true, true>(n, K, A, 1, si, alpha, C, ldc, row0, st);
+  return launch_gemm_atb_upper<true, true>(n, K, A, 1, si, alpha, C, ldc, row0, jmin, st);
 }
 
 cudaError_t rbmpp_trmv_upper(int n, const double* A, const double* x, double* y, cudaStream_t st) {
