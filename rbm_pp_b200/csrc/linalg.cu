@@ -99,6 +99,14 @@ __global__ void __launch_bounds__(256, BM > 64 ? 1 : 2) gemm_atb_upper(int n, in
   };
 #pragma unroll
   for (int st = 0; st < kStages - 1; st++) load(st);
+  // C's tile on its way to L2 while the products run: 16 rows of a column a line.  The smaller tiles are for few rows,
+  // whose C is there already.
+  if (ACC && BM == 128) {
+    for (int e = tid; e < BM * BM / 16; e += 256) {
+      const int i = i0 + 16 * (e % (BM / 16)), j = j0 + e / (BM / 16);
+      if (j < n && i <= j) asm volatile("prefetch.global.L2 [%0];" ::"l"(C + ldc * j + i));
+    }
+  }
   for (int st = 0; st < steps; st++) {
     asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
     __syncthreads();  // step st has landed everywhere, and everybody is done with the buffer refilled below
@@ -124,27 +132,42 @@ __global__ void __launch_bounds__(256, BM > 64 ? 1 : 2) gemm_atb_upper(int n, in
     }
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
+  // With ACC a batch of columns is loaded before any of it is stored (a store may alias the next column's loads, which
+  // would put a memory latency between columns).  With the prefetch above: split SR step of 10,404 parameters 55.7 ->
+  // 53.4 ms, FP64 step of 4,226 unchanged at 12.7 ms.
+  constexpr int BB = PJ > 3 ? 1 : PJ;  // what the registers hold
 #pragma unroll
-  for (int b = 0; b < PJ; b++)
+  for (int b0 = 0; b0 < PJ; b0 += BB) {
+    double old[BB][2][PI];
+    if (ACC) {
 #pragma unroll
-    for (int e = 0; e < 2; e++) {
-      const int j = j0 + wj + 8 * b + 2 * c + e;
-      if (j >= n || j < jmin) continue;
-      double* col = C + ldc * j;
-      double old[PI];
-      if (ACC) {
+      for (int b = 0; b < BB; b++)
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+          const int j = j0 + wj + 8 * (b0 + b) + 2 * c + e;
+          const double* col = C + ldc * j;
+#pragma unroll
+          for (int a = 0; a < PI; a++) {
+            const int i = i0 + wi + 8 * a + g;
+            old[b][e][a] = j < n && j >= jmin && i <= j ? col[i] : 0.0;
+          }
+        }
+    }
+#pragma unroll
+    for (int b = 0; b < BB; b++)
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const int j = j0 + wj + 8 * (b0 + b) + 2 * c + e;
+        if (j >= n || j < jmin) continue;
+        double* col = C + ldc * j;
 #pragma unroll
         for (int a = 0; a < PI; a++) {
           const int i = i0 + wi + 8 * a + g;
-          old[a] = i <= j ? col[i] : 0.0;
+          const double v = alpha * acc[a][b0 + b][e];
+          if (i <= j) col[i] = ACC ? old[b][e][a] + v : v;
         }
       }
-#pragma unroll
-      for (int a = 0; a < PI; a++) {
-        const int i = i0 + wi + 8 * a + g;
-        if (i <= j) col[i] = ACC ? old[a] + alpha * acc[a][b][e] : alpha * acc[a][b][e];
-      }
-    }
+  }
 }
 
 template <int BM, bool KCONTIG, bool ACC>
