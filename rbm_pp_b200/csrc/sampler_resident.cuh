@@ -383,6 +383,13 @@ __device__ __forceinline__ double recip(double b) {
   return fma(y, fma(-b, y, 1.0), y);
 }
 
+// a / b for any a and b, with y = recip(b).  Where b or the quotient is extreme the correction would overflow or lose
+// its residual (an infinite a y, for one, turns it into NaN): there the division.
+__device__ __forceinline__ double quotient(double a, double b, double y) {
+  const double ab = fabs(b), q = fabs(a * y);
+  return ab > 1e-250 && ab < 1e250 && q > 1e-30 && q < 1e30 ? div_by(a, b, y) : __ddiv_rn(a, b);
+}
+
 // grnd of one MT19937 word (mt.f:70-102): y / (2^32 - 1) rounded, equal to the division for every 32-bit y
 __device__ __forceinline__ double word_u(uint32_t y) {
   y ^= (y >> 11);
@@ -621,7 +628,7 @@ __device__ __forceinline__ void update_share(double* Y, const RMove& m, const Ga
   const int lane = threadIdx.x & 31, nr = r1 - r0;
   double* y = Y + r0 * LD;
   const double wvc = t[0] - t[4], Rr = t[1] * t[2] - t[3] * wvc;
-  const double inv_r1 = recip(t[1]), r1_over_r = t[1] * recip(Rr), wc = wvc * inv_r1;
+  const double inv_r1 = recip(t[1]), r1_over_r = quotient(t[1], Rr, recip(Rr)), wc = wvc * inv_r1;
   __syncwarp();
 #pragma unroll
   for (int q = 0; q < KPL; q++)
@@ -744,7 +751,7 @@ __device__ __forceinline__ void update_one(double* Y, const RMove& m, double v, 
   const double rho = Y[m.db * LD + kc], wv = warp_sum(pair_value<NP>(acc, v));
   __syncwarp();
   const double R1 = __shfl_sync(0xffffffffu, acc, m.ua), R = R1 * as[2 * m.db + 1] - ydbua * (wv - c);
-  const double inv_r1 = recip(R1), r1_over_r = div_by(R1, R, recip(R)), wc = (wv - c) * inv_r1;
+  const double inv_r1 = recip(R1), r1_over_r = quotient(R1, R, recip(R)), wc = (wv - c) * inv_r1;
   const double bk = (acc - (lane == m.ua ? 1.0 : 0.0)) * inv_r1, tk = (rho - ydbua * bk) * r1_over_r, cx = bk - wc * tk;
   // row batches: every load of a batch before its stores (a load cannot pass a store it may alias)
 #pragma unroll
@@ -1052,7 +1059,7 @@ __device__ __forceinline__ void resident_body(const DevDims& d, const DevTables&
       re = __shfl_sync(0xffffffffu, re, 0);
       im = d.cplx ? __shfl_sync(0xffffffffu, im, 0) : 0.0;
       const double num = __dadd_rn(abs_amp(re, im), d.shift);
-      const double r1a = (den > 1e-250 && den < 1e250) ? div_by(num, den, inv_den) : __ddiv_rn(num, den);
+      const double r1a = quotient(num, den, inv_den);
       const double uu = pub[par].u, r1sq = __dmul_rn(r1a, r1a);
       const bool ok = uu < r1sq;  // make_sample.f90:203-204
       have = ok ? sp1 : sp0;
