@@ -239,8 +239,16 @@ int rbmpp_set_replay(rbmpp_ctx* ctx, const int* decisions, int max_checkpoints);
  * what 1: walker 0 of the streaming sampler never issues its bulk load number `value` (1-based, 0 = off), so
  *         the consumer's bounded wait on it runs out: make_sample returns RBMPP_E_TIMEOUT and the context
  *         stays usable (the next make_sample rebuilds every walker's state);
- * what 2: poll bound of the streaming sampler's pipeline waits (0 = the default, 2^22 polls). */
+ * what 2: poll bound of the streaming sampler's pipeline waits (0 = the default, 2^22 polls).
+ * A context on which a hook has been set, to 0 as well, no longer takes the resident sampler. */
 int rbmpp_debug_hook(rbmpp_ctx* ctx, int what, int value);
+/* The sampler that rbmpp_make_sample takes for this context (tables set): direct (inverse blocks in global memory,
+ * updated at once), streaming (blocks streamed through shared memory, updates deferred), resident (blocks in
+ * shared memory for the whole call) or skew (transverse projection).  By shape, the resident one where the blocks
+ * fit, unless the environment variable RBMPP_SAMPLER was "stream" or "direct" at rbmpp_create, which leaves the streaming
+ * sampler where it applies or the direct one.  -1 for a null context. */
+enum { RBMPP_SAMPLER_DIRECT = 0, RBMPP_SAMPLER_STREAM = 1, RBMPP_SAMPLER_RESIDENT = 2, RBMPP_SAMPLER_SKEW = 3 };
+int rbmpp_sampler_kind(const rbmpp_ctx* ctx);
 
 /* Adjoint O_k kernel: for n configurations x(N, n): psi(0:N_QP, n) complex, hpsi(n) complex
  * (sum_x' <x|H|x'> psi(x'), calc_local_energy_correlation), and O(Nv, n) = d psi(x) / d theta_k

@@ -24,7 +24,7 @@ EXPORTS = ["rbmpp_create", "rbmpp_destroy", "rbmpp_last_error", "rbmpp_query", "
            "rbmpp_set_s_precision", "rbmpp_batch_create", "rbmpp_batch_destroy", "rbmpp_batch_last_error",
            "rbmpp_batch_tune", "rbmpp_batch_make_sample", "rbmpp_measure_correlation",
            "rbmpp_get_walker_events", "rbmpp_set_trace", "rbmpp_set_replay", "rbmpp_debug_hook",
-           "rbmpp_copy_state", "rbmpp_set_allreduce", "rbmpp_get_params_c"]
+           "rbmpp_copy_state", "rbmpp_set_allreduce", "rbmpp_get_params_c", "rbmpp_sampler_kind"]
 
 SR_FP64 = 0
 SR_SPLIT_BF16 = 1
@@ -113,6 +113,7 @@ def lib():
         L.rbmpp_set_trace.argtypes = [P, C.c_int]
         L.rbmpp_set_replay.argtypes = [P, P, C.c_int]
         L.rbmpp_debug_hook.argtypes = [P, C.c_int, C.c_int]
+        L.rbmpp_sampler_kind.argtypes = [P]
         L.rbmpp_copy_state.argtypes = [P, P]
         L.rbmpp_set_allreduce.argtypes = [P, ALLREDUCE_FN, P]
         L.rbmpp_eval_configs_noalloc.argtypes = [P, C.c_int, P, P, P, P]
@@ -311,6 +312,10 @@ class Context:
 
     def debug_hook(self, what: int, value: int):
         self._chk(lib().rbmpp_debug_hook(self.h, int(what), int(value)))
+
+    def sampler_kind(self) -> str:
+        """The sampler that make_sample takes for this context."""
+        return ("direct", "stream", "resident", "skew")[lib().rbmpp_sampler_kind(self.h)]
 
     def copy_state_from(self, other: "Context"):
         """Continue from other's sampling state, parameters and iteration bookkeeping."""

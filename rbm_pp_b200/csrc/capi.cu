@@ -184,7 +184,7 @@ struct rbmpp_ctx {
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   double stats[10] = {0};
   int stream_stages = 0;  // > 0: TMA-streamed sampler with this many stages
-  bool sampler_auto = true;  // RBMPP_SAMPLER did not choose the direct sampler
+  bool resident_ok = true;   // neither RBMPP_SAMPLER nor a verification hook asked for another sampler
   bool est_fits = true;   // the estimator's workspace fits in shared memory (tiles there or in global scratch)
   bool est_smem_tiles = true;  // ... with its tiles in shared memory
   double* d_SE = nullptr;  // Slater_Elm [qp][2N][2N] of the skew form (transverse projection)
@@ -432,9 +432,9 @@ int check_walker_status(rbmpp_ctx* c, const int* d_status, int n, const char* wh
 
 // Threads per block when the context samples with its inverse blocks resident in shared memory, else 0.  A walker
 // that fits is latency-bound and several times faster there than streamed or read from L2 (figures in
-// sampler_resident.cuh).  The verification hooks address the streaming sampler's pipeline, so they keep it.
+// sampler_resident.cuh).
 int resident_threads(const rbmpp_ctx* c) {
-  if (!c->sampler_auto || c->d.skip_load > 0 || c->d.wait_polls > 0) return 0;
+  if (!c->resident_ok) return 0;
   int maxsm = 0;
   if (cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->dims.device) != cudaSuccess) return 0;
   return rbmpp_resident_threads(c->d, maxsm);
@@ -512,10 +512,10 @@ int rbmpp_create(const rbmpp_dims* dims, rbmpp_ctx** out) {
   c->est_fits = (long long)rbmpp_estimator_smem_any(d, maxsm) <= maxsm;
   c->est_smem_tiles = (long long)rbmpp_estimator_smem(d, 256) <= maxsm;
   c->stream_stages = rbmpp_stream_stages(d, maxsm);
-  if (getenv("RBMPP_SAMPLER") && std::string(getenv("RBMPP_SAMPLER")) == "direct") {
-    c->stream_stages = 0;
-    c->sampler_auto = false;
-  }
+  const char* want = getenv("RBMPP_SAMPLER");
+  const bool direct = want && std::string(want) == "direct", stream = want && std::string(want) == "stream";
+  if (direct) c->stream_stages = 0;
+  c->resident_ok = !direct && !stream;
   if (d.alphac) c->stream_stages = 0;  // the streaming sampler carries real units only
   int r;
   const int N = d.N;
@@ -1527,7 +1527,15 @@ int rbmpp_debug_hook(rbmpp_ctx* c, int what, int value) {
     case 2: c->d.wait_polls = value; break;
     default: return fail(c, RBMPP_E_ARG, "unknown debug hook %d", what);
   }
+  c->resident_ok = false;  // the hooks address the streaming sampler, which has to recover from them
   return 0;
+}
+
+int rbmpp_sampler_kind(const rbmpp_ctx* c) {
+  if (!c) return -1;
+  if (c->d.skew) return RBMPP_SAMPLER_SKEW;
+  if (resident_threads(c)) return RBMPP_SAMPLER_RESIDENT;
+  return c->stream_stages > 0 ? RBMPP_SAMPLER_STREAM : RBMPP_SAMPLER_DIRECT;
 }
 
 int rbmpp_get_walker_events(const rbmpp_ctx* cc, int* events, double* trace) {
