@@ -478,13 +478,13 @@ cudaError_t launch_cor_fast(const DevDims& d, const DevTables& t, const DevParam
   return cudaGetLastError();
 }
 
-template <int KPL, int NP>
+template <int KPL>
 __device__ __forceinline__ void correlation_config(const DevDims& d, const DevTables& t, const DevParams& p,
                                                    const int8_t* xs, int n, double* out_psi, double* out_hpsi,
                                                    double* rows, double* sdr, int* out_nap, int* out_status,
                                                    const WS& s, const Cor& e, int cfgi) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int N = d.N, Np = NP > 0 ? NP : d.Np, ld = Np + 1, NB = 4 * N;
+  const int N = d.N, Np = d.Np, ld = Np + 1;
 
   for (int i = tid; i < N; i += blockDim.x) s.x[i] = (int)xs[(size_t)cfgi * N + i];
   for (int k = tid; k < Np * Np; k += blockDim.x) e.psx[k] = 0.0;
@@ -528,9 +528,9 @@ __device__ __forceinline__ void correlation_config(const DevDims& d, const DevTa
     if (warp < e.nqw && q0 + warp < d.n_qp) {
       const int qp = q0 + warp, mp = qp >> 1;
       double* T = e.tiles + (size_t)warp * Np * ld;
-      warp_gather_tile<KPL, NP, 8>(T, p.XF + (size_t)qp * N * N, s.idx, Np, N);
+      warp_gather_tile<KPL, 0, 8>(T, p.XF + (size_t)qp * N * N, s.idx, Np, N);
       bool sing;
-      const double det = warp_gj<KPL, NP, (KPL <= 2 ? 16 : (KPL <= 4 ? 8 : 4))>(T, Np, e.perm + (size_t)warp * Np, sing);
+      const double det = warp_gj<KPL, 0, (KPL <= 2 ? 16 : (KPL <= 4 ? 8 : 4))>(T, Np, e.perm + (size_t)warp * Np, sing);
       const double pfq = (double)d.pf_sign * det;
       const cplx cw = psi_wo_pf(d, t, s.rbm[qp], s.sgn[mp], qp);
       if (lane == 0) {
@@ -678,7 +678,7 @@ __global__ void fill_kernel(double* a, long long n, double v) {
     a[i] = v;
 }
 
-template <int KPL, int NP>
+template <int KPL>
 __global__ void __launch_bounds__(kCorThreads, 1)
     correlation_kernel(const __grid_constant__ DevDims d, const __grid_constant__ DevTables t,
                        const __grid_constant__ DevParams p, const int8_t* xs, int n, double* out_psi,
@@ -687,7 +687,7 @@ __global__ void __launch_bounds__(kCorThreads, 1)
   extern __shared__ __align__(16) char smem[];
   __shared__ WS s;
   __shared__ Cor e;
-  const int Np = NP > 0 ? NP : d.Np, ld = Np + 1;
+  const int Np = d.Np, ld = Np + 1;
   if (threadIdx.x == 0) {
     cor_layout(d, nqw, smem, &s, &e, gbuf != nullptr);
     if (gbuf) {
@@ -700,7 +700,7 @@ __global__ void __launch_bounds__(kCorThreads, 1)
   // one sample per block, or (global scratch) the samples blockIdx.x, blockIdx.x + gridDim.x, ...
   for (int cfgi = blockIdx.x; cfgi < n; cfgi += gridDim.x) {
     __syncthreads();
-    correlation_config<KPL, NP>(d, t, p, xs, n, out_psi, out_hpsi, rows, sdr, out_nap, out_status, s, e, cfgi);
+    correlation_config<KPL>(d, t, p, xs, n, out_psi, out_hpsi, rows, sdr, out_nap, out_status, s, e, cfgi);
   }
 }
 
@@ -760,22 +760,22 @@ cudaError_t rbmpp_launch_correlation(const DevDims& d, const DevTables& t, const
   }
   const int kpl = (d.Np + 31) / 32;
   cudaError_t rc = cudaErrorInvalidValue;
-#define LAUNCH(K, NPC)                                                                                          \
-  do {                                                                                                          \
-    rc = cudaFuncSetAttribute(correlation_kernel<K, NPC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-    if (rc == cudaSuccess) {                                                                                    \
-      rbmpp_note_launch();                                                                                      \
-      correlation_kernel<K, NPC><<<grid, kCorThreads, smem, st>>>(d, t, p, xs, n, out_psi, out_hpsi, rows, sdr,  \
-                                                                   out_nap, out_status, nqw, gbuf);              \
-      rc = cudaGetLastError();                                                                                  \
-    }                                                                                                           \
-    if (gbuf) cudaFreeAsync(gbuf, st);                                                                          \
-    return rc;                                                                                                  \
+#define LAUNCH(K)                                                                                             \
+  do {                                                                                                        \
+    rc = cudaFuncSetAttribute(correlation_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+    if (rc == cudaSuccess) {                                                                                  \
+      rbmpp_note_launch();                                                                                    \
+      correlation_kernel<K><<<grid, kCorThreads, smem, st>>>(d, t, p, xs, n, out_psi, out_hpsi, rows, sdr,    \
+                                                                   out_nap, out_status, nqw, gbuf);           \
+      rc = cudaGetLastError();                                                                                \
+    }                                                                                                         \
+    if (gbuf) cudaFreeAsync(gbuf, st);                                                                        \
+    return rc;                                                                                                \
   } while (0)
-  if (kpl <= 1) LAUNCH(1, 0);
-  if (kpl <= 2) LAUNCH(2, 0);
-  if (kpl <= 4) LAUNCH(4, 0);
-  if (kpl <= 8) LAUNCH(8, 0);
+  if (kpl <= 1) LAUNCH(1);
+  if (kpl <= 2) LAUNCH(2);
+  if (kpl <= 4) LAUNCH(4);
+  if (kpl <= 8) LAUNCH(8);
 #undef LAUNCH
   if (gbuf) cudaFreeAsync(gbuf, st);
   return rc;

@@ -622,13 +622,13 @@ cudaError_t launch_fast(const DevDims& d, const DevTables& t, const DevParams& p
   return cudaGetLastError();
 }
 
-template <int KPL, int NP>
+template <int KPL>
 __device__ __forceinline__ void estimator_config(const DevDims& d, const DevTables& t, const DevParams& p,
                                                  const int8_t* xs, int n, double* out_psi, double* out_hpsi,
                                                  double* O, int* out_nap, int* out_status, int reweight, const WS& s,
                                                  const Est& e, int cfgi) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int N = d.N, Np = NP > 0 ? NP : d.Np, ld = Np + 1, NB = 4 * N;
+  const int N = d.N, Np = d.Np, ld = Np + 1, NB = 4 * N;
   // complex projection weights: a real row and an imaginary row per configuration
   double* Orow = O ? O + (size_t)cfgi * d.Nv * (d.cplx ? 2 : 1) : nullptr;
   double* OrowI = (Orow && d.cplx) ? Orow + d.Nv : nullptr;
@@ -706,9 +706,9 @@ __device__ __forceinline__ void estimator_config(const DevDims& d, const DevTabl
       const int mp = qp >> 1, sp = qp & 1;
       const double* XFq = p.XF + (size_t)qp * N * N;
       const double* XFTq = p.XFT + (size_t)qp * N * N;
-      warp_gather_tile<KPL, NP, 8>(T, XFq, s.idx, Np, N);
+      warp_gather_tile<KPL, 0, 8>(T, XFq, s.idx, Np, N);
       bool sing;
-      const double det = warp_gj<KPL, NP, (KPL <= 2 ? 16 : (KPL <= 4 ? 8 : 4))>(T, Np, src, sing);
+      const double det = warp_gj<KPL, 0, (KPL <= 2 ? 16 : (KPL <= 4 ? 8 : 4))>(T, Np, src, sing);
       if (sing) bad = true;
       const double pfq = (double)d.pf_sign * det;
       const cplx cw = psi_wo_pf_s(d, t, s, s.sgn[mp], qp);
@@ -1007,7 +1007,7 @@ __device__ __forceinline__ void estimator_config(const DevDims& d, const DevTabl
   }
 }
 
-template <int KPL, int NP>
+template <int KPL>
 __global__ void __launch_bounds__(kEstThreads, 1)
     estimator_kernel(const __grid_constant__ DevDims d, const __grid_constant__ DevTables t,
                      const __grid_constant__ DevParams p, const int8_t* xs, int n, double* out_psi, double* out_hpsi,
@@ -1015,7 +1015,7 @@ __global__ void __launch_bounds__(kEstThreads, 1)
   extern __shared__ __align__(16) char smem[];
   __shared__ WS s;
   __shared__ Est e;
-  const int Np = NP > 0 ? NP : d.Np, ld = Np + 1;
+  const int Np = d.Np, ld = Np + 1;
   if (threadIdx.x == 0) {
     est_layout(d, nqw, smem, &s, &e, gtiles != nullptr);
     if (gtiles) {
@@ -1027,7 +1027,7 @@ __global__ void __launch_bounds__(kEstThreads, 1)
   // one configuration per block, or (global tiles) the configurations blockIdx.x, blockIdx.x + gridDim.x, ...
   for (int cfgi = blockIdx.x; cfgi < n; cfgi += gridDim.x) {
     __syncthreads();
-    estimator_config<KPL, NP>(d, t, p, xs, n, out_psi, out_hpsi, O, out_nap, out_status, reweight, s, e, cfgi);
+    estimator_config<KPL>(d, t, p, xs, n, out_psi, out_hpsi, O, out_nap, out_status, reweight, s, e, cfgi);
   }
 }
 
@@ -1106,22 +1106,22 @@ cudaError_t rbmpp_launch_estimator(const DevDims& d, const DevTables& t, const D
   }
   int kpl = (d.Np + 31) / 32;
   cudaError_t rc = cudaErrorInvalidValue;
-#define LAUNCH(K, NPC)                                                                                     \
-  do {                                                                                                     \
-    rc = cudaFuncSetAttribute(estimator_kernel<K, NPC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-    if (rc == cudaSuccess) {                                                                               \
-      rbmpp_note_launch();                                                                                 \
-      estimator_kernel<K, NPC><<<grid, kEstThreads, smem, st>>>(d, t, p, xs, n, out_psi, out_hpsi, O, out_nap, \
+#define LAUNCH(K)                                                                                           \
+  do {                                                                                                      \
+    rc = cudaFuncSetAttribute(estimator_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+    if (rc == cudaSuccess) {                                                                                \
+      rbmpp_note_launch();                                                                                  \
+      estimator_kernel<K><<<grid, kEstThreads, smem, st>>>(d, t, p, xs, n, out_psi, out_hpsi, O, out_nap,   \
                                                                 out_status, reweight, nqw, gtiles);         \
-      rc = cudaGetLastError();                                                                             \
-    }                                                                                                      \
-    if (gtiles) cudaFreeAsync(gtiles, st);                                                                 \
-    return rc;                                                                                             \
+      rc = cudaGetLastError();                                                                              \
+    }                                                                                                       \
+    if (gtiles) cudaFreeAsync(gtiles, st);                                                                  \
+    return rc;                                                                                              \
   } while (0)
-  if (kpl <= 1) LAUNCH(1, 0);
-  if (kpl <= 2) LAUNCH(2, 0);
-  if (kpl <= 4) LAUNCH(4, 0);
-  if (kpl <= 8) LAUNCH(8, 0);
+  if (kpl <= 1) LAUNCH(1);
+  if (kpl <= 2) LAUNCH(2);
+  if (kpl <= 4) LAUNCH(4);
+  if (kpl <= 8) LAUNCH(8);
 #undef LAUNCH
   if (gtiles) cudaFreeAsync(gtiles, st);
   return rc;

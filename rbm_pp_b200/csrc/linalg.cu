@@ -66,7 +66,7 @@ __device__ __forceinline__ void load_operand(double* dst, const double* __restri
 }
 
 template <int BM, bool KCONTIG, bool ACC, int VEC>
-__global__ void __launch_bounds__(256, BM > 64 ? 1 : 2) gemm_atb_upper(int n, int K, const double* __restrict__ A, long long sk,
+__global__ void __launch_bounds__(256, 1) gemm_atb_upper(int n, int K, const double* __restrict__ A, long long sk,
                                                          long long si, double alpha, double* __restrict__ C,
                                                          long long ldc, int row0, int jmin) {
   // upper-tile index -> (ti, tj) with ti <= tj
@@ -99,8 +99,8 @@ __global__ void __launch_bounds__(256, BM > 64 ? 1 : 2) gemm_atb_upper(int n, in
   };
 #pragma unroll
   for (int st = 0; st < kStages - 1; st++) load(st);
-  // C's tile on its way to L2 while the products run: 16 rows of a column a line.  The smaller tiles are for few rows,
-  // whose C is there already.
+  // C's tile on its way to L2 while the products run: 16 rows of a column a line.  The smaller tiles are mostly for few
+  // rows, whose C is there already.
   if (ACC && BM == 128) {
     for (int e = tid; e < BM * BM / 16; e += 256) {
       const int i = i0 + 16 * (e % (BM / 16)), j = j0 + e / (BM / 16);
@@ -185,9 +185,9 @@ cudaError_t launch_gemm_bm(int n, int K, const double* A, long long sk, long lon
 }
 
 // The tile size with the least time by waves of whole tiles: a wave of 96-wide tiles takes 0.6 of one of 128-wide ones
-// (0.56 of the products, at slightly more loads for each), two 64-wide tiles to an SM 0.6 too (half the products, at
-// twice the loads).  A last wave that is nearly empty (595 tiles of 128 at 4226 rows: four waves and three tiles)
-// or a matrix of few tiles is what the smaller sizes are for.
+// (0.56 of the products, at slightly more loads for each).  That avoids a last wave that is nearly empty (595 tiles
+// of 128 at 4226 rows: four waves and three tiles), and a matrix of one wave has more, smaller tiles: on 148 SMs
+// every n up to 1536 takes 96.
 template <bool KCONTIG, bool ACC>
 cudaError_t launch_gemm_atb_upper(int n, int K, const double* A, long long sk, long long si, double alpha, double* C,
                                   long long ldc, int row0, int jmin, cudaStream_t st) {
@@ -195,14 +195,13 @@ cudaError_t launch_gemm_atb_upper(int n, int K, const double* A, long long sk, l
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return e;
-  auto waves = [&](int bm, int slots) {
+  auto waves = [&](int bm) {
     const long long nt = (n - row0 + bm - 1) / bm, tiles = nt * (nt + 1) / 2;
-    return (double)((tiles + slots - 1) / slots);
+    return (double)((tiles + nsm - 1) / nsm);
   };
-  const double t128 = waves(128, nsm), t96 = 0.6 * waves(96, nsm), t64 = 0.6 * waves(64, 2 * nsm);
-  if (t128 <= t96 && t128 <= t64) return launch_gemm_bm<128, KCONTIG, ACC>(n, K, A, sk, si, alpha, C, ldc, row0, jmin, st);
-  if (t96 <= t64) return launch_gemm_bm<96, KCONTIG, ACC>(n, K, A, sk, si, alpha, C, ldc, row0, jmin, st);
-  return launch_gemm_bm<64, KCONTIG, ACC>(n, K, A, sk, si, alpha, C, ldc, row0, jmin, st);
+  return waves(128) <= 0.6 * waves(96)
+             ? launch_gemm_bm<128, KCONTIG, ACC>(n, K, A, sk, si, alpha, C, ldc, row0, jmin, st)
+             : launch_gemm_bm<96, KCONTIG, ACC>(n, K, A, sk, si, alpha, C, ldc, row0, jmin, st);
 }
 
 // mirror the upper triangle into the lower one
