@@ -6,30 +6,13 @@
 // reads and writes the whole tile.  Here the tile lives in the warp's registers, rows over eight lane groups and
 // columns over four, so a step moves one column and one row through shared memory.
 #pragma once
+#include "fp64_ops.cuh"
 #include "walker_ops.cuh"
 
 namespace {
 
 // Row length of a tile in doubles: 4 mod 16, so that the 8 x 4 fragments of the matrix units fall on distinct banks
 constexpr int tile_ld(int np) { return (np + 11) / 16 * 16 + 4; }
-
-// 1 / b by Newton's iteration from the hardware's approximation; b = 0, infinite or extreme: the division (which is
-// a call of some 300 cycles, on the critical path of every elimination step)
-__device__ __forceinline__ double newton_recip(double b) {
-  const double ab = fabs(b);
-  if (!(ab > 1e-280 && ab < 1e280)) return 1.0 / b;
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-  y = fma(y, fma(-b, y, 1.0), y);
-  y = fma(y, fma(-b, y, 1.0), y);
-  return fma(y, fma(-b, y, 1.0), y);
-}
-
-__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
-  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-      : "+d"(c[0]), "+d"(c[1])
-      : "d"(a), "d"(b));
-}
 
 // Shared memory of one warp: pivot column and row of two successive steps, the pivot rows, their inverse map and the
 // reciprocal pivots
@@ -93,7 +76,7 @@ __device__ __forceinline__ double reg_inverse(double* T, InvBuf<NP>& w, bool& si
         const bool up = NP > 32 && v1 > v0;
         const double v = up ? v1 : v0, x = up ? x1 : x0;
         const unsigned hi = (unsigned)__double2hiint(v), mh = __reduce_max_sync(0xffffffffu, hi);
-        const double y = newton_recip(v > 0.0 ? x : 1.0);  // of every lane's candidate, while the search runs
+        const double y = recip(v > 0.0 ? x : 1.0);  // of every lane's candidate, while the search runs
         bool best = hi == mh;
         const unsigned m = __ballot_sync(0xffffffffu, best);
         if (mh == 0u || (m & (m - 1u))) {  // the upper halves tie

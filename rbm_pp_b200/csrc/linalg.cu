@@ -5,6 +5,9 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "fp64_ops.cuh"
+#include "tma.cuh"
+
 void rbmpp_note_launch();  // capi.cu: counts kernel launches
 
 namespace {
@@ -27,15 +30,6 @@ template <int BM, bool KCONTIG>
 constexpr int kTileDoubles = KCONTIG ? BM * kLdK : BK * (BM + 4);
 template <int BM, bool KCONTIG>
 constexpr int kGemmSmem = kStages * 2 * kTileDoubles<BM, KCONTIG> * 8;
-
-__device__ __forceinline__ void cp_async16(void* dst, const void* src, int bytes) {
-  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void cp_async8(void* dst, const void* src, int bytes) {
-  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
-}
 
 // One operand tile: k0 .. k0 + BK of columns i0 .. i0 + BM; zeros beyond K and n
 template <int BM, bool KCONTIG, int VEC>
@@ -95,7 +89,7 @@ __global__ void __launch_bounds__(256, 1) gemm_atb_upper(int n, int K, const dou
       load_operand<BM, KCONTIG, VEC>(p, A, sk, si, n, K, i0, st * BK);
       load_operand<BM, KCONTIG, VEC>(p + TD, A, sk, si, n, K, j0, st * BK);
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");
+    cp_async_commit();
   };
 #pragma unroll
   for (int st = 0; st < kStages - 1; st++) load(st);
@@ -108,7 +102,7 @@ __global__ void __launch_bounds__(256, 1) gemm_atb_upper(int n, int K, const dou
     }
   }
   for (int st = 0; st < steps; st++) {
-    asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
+    cp_async_wait<kStages - 2>();
     __syncthreads();  // step st has landed everywhere, and everybody is done with the buffer refilled below
     load(st + kStages - 1);
     const double* As = sm + (st % kStages) * 2 * TD;
@@ -126,12 +120,10 @@ __global__ void __launch_bounds__(256, 1) gemm_atb_upper(int n, int K, const dou
       for (int a = 0; a < PI; a++)
 #pragma unroll
         for (int b = 0; b < PJ; b++)
-          asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-              : "+d"(acc[a][b][0]), "+d"(acc[a][b][1])
-              : "d"(fa[a]), "d"(fb[b]));
+          dmma(acc[a][b], fa[a], fb[b]);
     }
   }
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  cp_async_wait<0>();
   // With ACC a batch of columns is loaded before any of it is stored (a store may alias the next column's loads, which
   // would put a memory latency between columns).  With the prefetch above: split SR step of 10,404 parameters 55.7 ->
   // 53.4 ms, FP64 step of 4,226 unchanged at 12.7 ms.

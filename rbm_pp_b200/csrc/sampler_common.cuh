@@ -1,5 +1,6 @@
-// sampler_common.cuh -- walker-level routines shared by the two sampler kernels (sampler.cu: immediate
-// rank-2 updates; sampler_stream.cu: TMA-streamed projections with deferred updates).
+// sampler_common.cuh -- walker-level routines shared by the sampler kernels (sampler.cu: immediate
+// rank-2 updates; sampler_stream.cu: TMA-streamed projections with deferred updates; sampler_resident.cuh: inverses in
+// shared memory; skew.cu: the full skew form).
 #pragma once
 #include "tma.cuh"
 #include "walker_ops.cuh"

@@ -21,6 +21,7 @@
 // Inverses from scratch work in place in the resident tiles; the walker's slice of DevWalkers::Y in global memory
 // only keeps the old tiles for the drift test and for a rejected global flip.
 #pragma once
+#include "fp64_ops.cuh"
 #include "sampler_common.cuh"
 
 namespace {
@@ -365,38 +366,13 @@ __device__ __noinline__ void res_flip(const SCtx& c) {
 
 // ---- control warp ------------------------------------------------------------------------------------------
 
-// a / b from y, an approximation of 1 / b: the quotient a y and one residual correction (Markstein 1990), which is
-// the rounded quotient when y is the rounded reciprocal and no exponent is extreme.  CUDA's division is a call of
-// some 300 cycles, and several of them stood one after another on the critical path of a proposal.
-__device__ __forceinline__ double div_by(double a, double b, double y) {
-  const double q = a * y;
-  return fma(fma(-q, b, a), y, q);
-}
-// 1 / b by Newton's iteration from the hardware's approximation; b = 0, infinite or extreme: the division
-__device__ __forceinline__ double recip(double b) {
-  const double ab = fabs(b);
-  if (!(ab > 1e-280 && ab < 1e280)) return 1.0 / b;
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-  y = fma(y, fma(-b, y, 1.0), y);
-  y = fma(y, fma(-b, y, 1.0), y);
-  return fma(y, fma(-b, y, 1.0), y);
-}
-
-// a / b for any a and b, with y = recip(b).  Where b or the quotient is extreme the correction would overflow or lose
-// its residual (an infinite a y, for one, turns it into NaN): there the division.
-__device__ __forceinline__ double quotient(double a, double b, double y) {
-  const double ab = fabs(b), q = fabs(a * y);
-  return ab > 1e-250 && ab < 1e250 && q > 1e-30 && q < 1e30 ? div_by(a, b, y) : __ddiv_rn(a, b);
-}
-
-// grnd of one MT19937 word (mt.f:70-102): y / (2^32 - 1) rounded, equal to the division for every 32-bit y
+// grnd of one MT19937 word (mt.f:70-102)
 __device__ __forceinline__ double word_u(uint32_t y) {
   y ^= (y >> 11);
   y ^= (y << 7) & 0x9d2c5680u;
   y ^= (y << 15) & 0xefc60000u;
   y ^= (y >> 18);
-  return div_by((double)y, 4294967295.0, 1.0 / 4294967295.0);
+  return word_fraction(y);
 }
 
 // the next block of the generator (the recurrence of mt_next): 32 words at a time, each group reading words that no

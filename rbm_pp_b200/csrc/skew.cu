@@ -391,14 +391,13 @@ __device__ __forceinline__ void warp_gxy(const double* Gq, const double* xh, con
 template <int N>
 __device__ __forceinline__ void fetch_tile(double* buf, const double* Gq) {
   __syncwarp();
-  const uint32_t dst = smem_u32(buf);
 #pragma unroll 4
   for (int e = threadIdx.x & 31; e < N * N / 2; e += 32)
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * e), "l"(Gq + 2 * e) : "memory");
-  asm volatile("cp.async.commit_group;" ::: "memory");
+    cp_async16(buf + 2 * e, Gq + 2 * e, 16);
+  cp_async_commit();
 }
 __device__ __forceinline__ void fetch_wait() {
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  cp_async_wait<0>();
   __syncwarp();
 }
 

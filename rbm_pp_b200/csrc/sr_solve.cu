@@ -15,6 +15,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "fp64_ops.cuh"
 #include "tma.cuh"
 
 void rbmpp_note_launch();  // capi.cu: counts kernel launches
@@ -70,23 +71,6 @@ __device__ __forceinline__ void load_block(int nb, const double* __restrict__ A,
 // 8 x 4 fragments on distinct banks and the 32-row pieces on 16-byte boundaries.
 // ---------------------------------------------------------------------------------------------------
 constexpr int LB = NB + 4;
-
-__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
-  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-      : "+d"(c[0]), "+d"(c[1])
-      : "d"(a), "d"(b));
-}
-
-// 1 / sqrt(d) by Newton's iteration from the hardware's approximation (extreme d: the division)
-__device__ __forceinline__ double newton_rsqrt(double d) {
-  if (!(d > 1e-280 && d < 1e280)) return 1.0 / sqrt(d);
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-  const double h = 0.5 * d;
-#pragma unroll
-  for (int i = 0; i < 3; i++) y = fma(y, fma(-h * y, y, 0.5), y);
-  return y;
-}
 
 // x <- U^{-T} x for one column x of 32 rows, one thread: U (32 x 32, upper) at Ud, its reciprocal diagonal at rd
 __device__ __forceinline__ void solve_column32(const double* Ud, const double* rd, double* x) {
@@ -225,12 +209,11 @@ __global__ void __launch_bounds__(512, 1)
             if (lane == 0 && *info == 0) *info = k0 + p0 + k + 1;
             dkk = 1.0;
           }
-          const double rk = newton_rsqrt(dkk);
-          double ukk = dkk * rk;
+          double rk;
+          const double ukk = sqrt_recip(dkk, rk);
           // row k of U: U(k, c) = T(k, c) / U(k, k) in lane c > k
           double ukc = col[k] * rk;
           if (k + 1 < 32) next = __shfl_sync(0xffffffffu, fma(-ukc, ukc, col[k + 1 < 32 ? k + 1 : 31]), (k + 1) & 31);
-          ukk = fma(fma(-ukk, ukk, dkk), 0.5 * rk, ukk);
           if (lane == 0) rdiag[p0 + k] = rk;
           if (lane == k) ukc = ukk;
           col[k] = ukc;

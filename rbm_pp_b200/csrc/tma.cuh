@@ -1,5 +1,5 @@
-// tma.cuh -- thin wrappers over the sm_90+/sm_100a bulk-copy (TMA, non-tensor) and mbarrier PTX used by
-// the streaming sampler.  No multicast form is used anywhere.
+// tma.cuh -- thin wrappers over the asynchronous-copy PTX: the sm_90+/sm_100a bulk copies (TMA, non-tensor) and
+// mbarriers, and the per-thread cp.async.  No multicast form is used anywhere.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -63,3 +63,17 @@ __device__ __forceinline__ void bulk_wait_read_all() { asm volatile("cp.async.bu
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 // order async-proxy global writes with later generic-proxy accesses
 __device__ __forceinline__ void fence_proxy_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
+
+// global -> shared copies of one thread: 16 bytes past L1, or 8; the words past `bytes` are zeros
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async8(void* dst, const void* src, int bytes) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// all but the thread's last `left` groups have landed
+template <int left>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(left) : "memory");
+}
