@@ -187,9 +187,10 @@ BATCH_J2 = (0.40, 0.45, 0.50, 0.55, 0.60)
 
 def run_batch(args):
     """Batched sampling over lattices L = 12..18 crossed with J2/J1 = 0.40..0.60 (1024 walkers each,
-    alpha = 2, no translation projection, N_QP = 2): one persistent launch per make_sample, launch shape
-    and walker order picked by the autotuner.  Reports aggregate MC samples/s of the batched launch and,
-    for comparison, each instance's MC samples/s when launched alone."""
+    alpha = 2, no translation projection, N_QP = 2): one call per make_sample, which launches the walkers resident in
+    shared memory (L = 12, 14) beside those of the direct sampler (L = 16, 18), launch shape and walker order picked by
+    the autotuner.  Reports aggregate MC samples/s of the batch and, for comparison, each instance's MC samples/s
+    from its own make_sample."""
     import torch
     from rbm_pp_b200 import capi
     from rbm_pp_b200 import formats as fm
@@ -219,15 +220,13 @@ def run_batch(args):
     clocks = clk.stop()
     batch_ms = float(np.mean(ms))
     total_samples = walkers * ns * len(ctxs)
-    # each instance alone (same direct sampler), one make_sample each
-    os.environ["RBMPP_SAMPLER"] = "direct"
-    alone = []
+    alone = []  # each instance's own make_sample, by the sampler of its shape
     for g, (L, J2) in zip(ctxs, meta):
         g.make_sample(False)
         t = g.stats()["sampler_ms"]
-        alone.append({"L": L, "J2": J2, "ms": t, "samples_per_s": walkers * ns / (t * 1e-3)})
-    os.environ.pop("RBMPP_SAMPLER", None)
-    line = {"metric": "MC samples/s, batched lattices L=12..18 x J2/J1=0.40..0.60 in one launch",
+        alone.append({"L": L, "J2": J2, "sampler": g.sampler_kind(), "ms": t,
+                      "samples_per_s": walkers * ns / (t * 1e-3)})
+    line = {"metric": "MC samples/s, batched lattices L=12..18 x J2/J1=0.40..0.60 in one call",
             "value": total_samples / (batch_ms * 1e-3), "unit": "MC samples/s", "n_gpus": 1, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": batch_ms, "higher_is_better": True, "scaling": "weak",
             "vs_baseline": None, "dtype": "f64", "data": "synthetic (seeded, reference file shapes)",
@@ -247,8 +246,7 @@ def run_batch(args):
 
 def corr_flops_per_sample(w):
     """Algorithmic FP64 flops of one correlation-measured sample, per projection: the scratch inverse
-    (2 Np^3), one mat-vec W = Y v per up electron (2 Np^3) and two dot products of length Np per
-    up-down pair (4 Np^3)."""
+    (2 Np^3) and three Np x Np x Np products, whose elements give the ratios of all up-down pairs (6 Np^3)."""
     np_ = w["L"] ** 2 // 2
     n_qp = 2 * (w["L"] ** 2 if w["translations"] else 1)
     return n_qp * 8.0 * np_ ** 3
@@ -294,7 +292,7 @@ def run_corr(args):
                        "alphar": w["alphar"], "n_qp": 2 * (w["L"] ** 2 if w["translations"] else 1),
                        "l2": "per-sample rows larger than L2"},
             "kernel_ms": kern_ms,
-            "roofline": {"kernel": "correlation_kernel", "bound": "fp64", "achieved": achieved, "peak": 40.0,
+            "roofline": {"kernel": "correlation_fast_kernel", "bound": "fp64", "achieved": achieved, "peak": 40.0,
                          "unit": "TFLOP/s", "frac": achieved / 40.0,
                          "peak_kind": "nominal FP64 (no measured FP64 peak on this pool)", "traffic": None,
                          "algorithmic_flops": flops},
@@ -319,6 +317,29 @@ def run_corr(args):
     print(json.dumps(line), flush=True)
     g.close()
     return 0
+
+
+def sampler_roofline(kind, n_qp, Np, proposals, accepts, ms):
+    """The roofline entry of one make_sample.  Streamed and direct: every proposal reads each projection's inverse block
+    (8 Np^2 bytes) from global memory and an accepted move reads and writes it again.  Resident: the blocks stay in
+    shared memory and a walker is a serial chain, so its FP64 rate (2 Np^2 flop per projection for the ratio, 6 Np^2 for
+    Y v and the rank-2 update) says how far the latency of its links leaves it from the arithmetic."""
+    if kind == "resident":
+        flops = n_qp * Np * Np * (2.0 * proposals + 6.0 * accepts)
+        achieved = flops / (ms * 1e-3) / 1e12
+        return {"kernel": "sampler_resident_kernel (make_sample)", "bound": "latency", "achieved": achieved, "peak": 40.0,
+                "unit": "TFLOP/s", "frac": achieved / 40.0,
+                "peak_kind": "nominal FP64 (no measured FP64 peak on this pool)", "traffic": None,
+                "algorithmic_flops": flops}
+    peaks, peak_kind = measured_peaks()
+    alg_bytes = n_qp * Np * Np * (8.0 * proposals + 16.0 * accepts)
+    achieved = alg_bytes / (ms * 1e-3) / 1e9
+    traffic = alg_bytes * SAMPLER_TRAFFIC_PER_ALG_BYTE if SAMPLER_TRAFFIC_PER_ALG_BYTE and kind == "stream" else None
+    return {"kernel": {"stream": "sampler_stream_kernel", "direct": "sampler_kernel"}[kind] + " (make_sample)",
+            "bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
+            "frac": achieved / peaks["hbm_gbs"], "peak_kind": peak_kind + " (burst copy)", "traffic": traffic,
+            "traffic_source": "ncu dram bytes / algorithmic bytes of the 1-wave capture, scaled" if traffic else None,
+            "algorithmic_bytes": alg_bytes}
 
 
 def run_ours(args):
@@ -411,14 +432,10 @@ def run_ours(args):
                                       "of_the_mean": abs(float(np.mean(energies[:n_pair])) - float(np.mean(pe)))
                                       / (w["L"] ** 2)}}
         twin.close()
-    peaks, peak_kind = measured_peaks()
     Np = (w["L"] ** 2) // 2
     n_qp = 2 * (w["L"] ** 2 if w["translations"] else 1)
-    bytes_prop = n_qp * 8.0 * Np * Np
-    bytes_acc = n_qp * 16.0 * Np * Np
-    alg_bytes = float(np.mean(props)) * bytes_prop + float(np.mean(acc_all)) * bytes_acc
     smp = float(np.mean(samp_ms))
-    achieved = alg_bytes / (smp * 1e-3) / 1e9
+    roofline = sampler_roofline(ctx.sampler_kind(), n_qp, Np, float(np.mean(props)), float(np.mean(acc_all)), smp)
     line = {"metric": METRIC, "value": value, "unit": "MC samples/s", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True, "scaling": "weak",
             "vs_baseline": None, "dtype": "f64", "data": "synthetic (seeded, reference file shapes)",
@@ -432,13 +449,7 @@ def run_ours(args):
             "phases_ms": {"make_sample": smp, "estimator": float(np.mean(est_ms)), "s_build": float(np.mean(sb_ms)),
                           "cholesky_solve": float(np.mean(solve_ms)), "refinement": float(np.mean(ref_ms)),
                           "sr_phase": float(np.mean(sb_ms)) + float(np.mean(solve_ms)) + float(np.mean(ref_ms))},
-            "roofline": {"kernel": "sampler_stream_kernel (make_sample)", "bound": "hbm", "achieved": achieved,
-                         "peak": peaks["hbm_gbs"], "unit": "GB/s", "frac": achieved / peaks["hbm_gbs"],
-                         "peak_kind": peak_kind + " (burst copy)",
-                         "traffic": (alg_bytes * SAMPLER_TRAFFIC_PER_ALG_BYTE if SAMPLER_TRAFFIC_PER_ALG_BYTE
-                                     else None),
-                         "traffic_source": "ncu dram bytes / algorithmic bytes of the 1-wave capture, scaled",
-                         "algorithmic_bytes": alg_bytes},
+            "roofline": roofline,
             "clocks": clocks,
             "e2e": {"value": e2e_v, "unit": "MC samples/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
             "gpu_launches": launches,
