@@ -430,9 +430,15 @@ int check_walker_status(rbmpp_ctx* c, const int* d_status, int n, const char* wh
   return 0;
 }
 
-// Threads per block when the context samples with its inverse blocks resident in shared memory, else 0.  A walker
-// that fits is latency-bound and several times faster there than streamed or read from L2 (figures in
-// sampler_resident.cuh).
+// Threads per block when the context samples with its inverse blocks resident in shared memory, else 0.  Wherever
+// they fit, because a walker there is faster at every number of walkers.  make_sample of two samples per walker, streamed
+// or direct -> resident, ms:      8 walkers       148            1,024           4,096
+//   4x4, 2 projections          2.8 -> 1.0    3.0 -> 1.0     20 -> 2.5       80 -> 8.7   (16,384: 315 -> 34)
+//   6x6, 72 projections          49 -> 17      49 -> 18     341 -> 122    1,359 -> 483
+//   8x8, 2 projections           13 -> 4.9     13 -> 5.2     91 -> 14       359 -> 51
+//   10x10, 2 projections         22 -> 13      25 -> 15     163 -> 67       642 -> 236
+//   12x12, 2 projections         92 -> 35      97 -> 38     643 -> 159
+//   14x14, 2 projections        350 -> 74     378 -> 79   2,502 -> 527
 int resident_threads(const rbmpp_ctx* c) {
   if (!c->resident_ok) return 0;
   int maxsm = 0;

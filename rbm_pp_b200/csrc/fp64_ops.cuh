@@ -1,10 +1,10 @@
-// fp64_ops.cuh -- scalar FP64 operations on the critical paths of the samplers, the register inverse and the Cholesky,
-// and the FP64 matrix product of a warp.
+// fp64_ops.cuh -- scalar FP64 operations on the critical paths of the samplers, the register inverse and the
+// Cholesky, and the FP64 matrix product of a warp.
 //
 // CUDA's double division, reciprocal and square root are calls of some 300 cycles; a proposal or an elimination step has
 // several of them one after another.  The forms below start from the hardware's approximation (PTX rcp.approx and
-// rsqrt.approx, about 20 bits), take three Newton steps and correct by the residual, which fma gives exactly.  Where an exponent is so
-// extreme that a step could overflow or lose its residual, they call CUDA's operation.
+// rsqrt.approx, about 20 bits), take three Newton steps and correct by the residual, which fma gives exactly.  Where
+// an exponent is so extreme that a step could overflow or lose its residual, they call CUDA's operation.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -61,8 +61,8 @@ __device__ __forceinline__ double word_fraction(uint32_t y) {
   return div_by((double)y, 4294967295.0, 1.0 / 4294967295.0);
 }
 
-// c += A B on the FP64 matrix units, 8 x 8 by one warp over four k: lane (g, t) = (lane / 4, lane % 4) gives A(g, t) and
-// B(t, g) and holds c[e] = C(g, 2 t + e)
+// c += A B on the FP64 matrix units, 8 x 8 by one warp over four k: lane (g, t) = (lane / 4, lane % 4) gives A(g, t)
+// and B(t, g) and holds c[e] = C(g, 2 t + e)
 __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
   asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
       : "+d"(c[0]), "+d"(c[1])

@@ -15,8 +15,9 @@
 //    it and, after an accepted move, the rank-2 update.
 //
 // Measured (B200, one make_sample; before: streamed, or the direct sampler reading Y from L2): 4x4, 8 walkers x 128
-// samples, 13.3 -> 4.7 ms; 6x6 with 72 projections, 256 walkers x 16, 139 -> 51 ms; 12x12, 256 walkers x 4, 198 ->
-// 46 ms; 75 walkers each of 12x12 and 14x14 in one batch, 377 -> 81 ms.
+// samples, 13.3 -> 4.7 ms; 6x6 with 72 projections, 256 walkers x 16, 139 -> 52 ms; 12x12, 256 walkers x 4, 198 ->
+// 47 ms (46 to 48 over 18 calls of three seeds; 148 walkers 41 ms: two walkers share an SM, and a launch takes as long
+// as its slowest walker); 75 walkers each of 12x12 and 14x14 in one batch, 377 -> 81 ms.
 //
 // Inverses from scratch work in place in the resident tiles; the walker's slice of DevWalkers::Y in global memory
 // only keeps the old tiles for the drift test and for a rejected global flip.
