@@ -41,12 +41,13 @@ constexpr int rows_update(int N) { return N == 36 ? 6 : N == 100 ? 5 : 8; }
 
 // A walker's block, or its cluster of blocks: every block carries the whole walker state (one random sequence, the same
 // decisions from the same numbers) and owns every size-th projection, so a G is touched by one block only.  What the
-// blocks exchange: the Pfaffians and drift of a from-scratch pass, and every proposal's partial sums.
+// blocks exchange: the Pfaffians and drift of a from-scratch pass, and every proposal's Pfaffians and
+// amplitudes.
 constexpr int kMaxCluster = 8;
+constexpr int kPsiSums = 8;  // partial sums of psi (sampler_skew_kernel)
 struct Team {
   int rank, size;
-  double* slots;  // shared, with size > 1: [2][size * warps][2] partial sums by parity of the proposal, then [size][2]
-  __device__ __forceinline__ int nwarps() const { return blockDim.x >> 5; }
+  double* slots;  // shared, with size > 1: [2][3 n_qp] Pfaffians and amplitudes by parity of the proposal, then [size][2]
   // the i-th projection that this block owns
   __device__ __forceinline__ int own(int i) const { return i * size + rank; }
   // barrier of all threads of the walker, with the memory order of __syncthreads over the cluster
@@ -80,7 +81,7 @@ __device__ __forceinline__ Team team(double* slots) {
   return m;
 }
 // doubles of Team::slots: they lie in the per-warp vectors of the block form, which the skew form does not use
-__host__ __device__ __forceinline__ int team_slots(int nwarps, int size) { return 4 * size * nwarps + 2 * size; }
+__host__ __device__ __forceinline__ int team_slots(int n_qp, int size) { return 6 * n_qp + 2 * size; }
 
 __device__ __forceinline__ int rho_of(const int* idx, int e, int Np, int N) { return idx[e] + (e >= Np ? N : 0); }
 
@@ -306,7 +307,7 @@ struct SkewScratch {
         if (s.red[32 + w] != 0.0 && !b) b = (int)s.red[32 + w];
       }
       if (m.size > 1) {
-        double* part = m.slots + 4 * m.size * m.nwarps();
+        double* part = m.slots + 6 * d.n_qp;
         m.put(part + 2 * m.rank, di);
         m.put(part + 2 * m.rank + 1, (double)b);
       } else {
@@ -317,7 +318,7 @@ struct SkewScratch {
     m.sync();
     if (m.size > 1) {
       if (threadIdx.x == 0) {
-        const double* part = m.slots + 4 * m.size * m.nwarps();
+        const double* part = m.slots + 6 * d.n_qp;
         double di = -1.0;
         int b = 0;
         for (int r = 0; r < m.size; r++) {
@@ -436,7 +437,8 @@ __device__ __forceinline__ double warp_skew_ratio(const DevDims& d, const DevPar
   xgy = warp_sum(xgy);
   const double gab = Gq[(size_t)a * N + b];
   __syncwarp();
-  return -gab * (ya + xgy) + gxa * gyb - gxb * gya;
+  // -G_ab (y_a + x^ . G y^) + (G x^)_a (G y^)_b - (G x^)_b (G y^)_a
+  return __fma_rn(-gxb, gya, __fma_rn(gxa, gyb, -__dmul_rn(gab, __dadd_rn(ya, xgy))));
 }
 
 // G' = G + V K^{-1} V^T after the accepted exchange, from Gq (global, or the warp's shared buffer) to Go (global);
@@ -489,7 +491,7 @@ __device__ __forceinline__ void warp_skew_update(const DevDims& d, const DevPara
   __syncwarp();
   // K = U^T G U - J (skew): upper entries
   const double k01 = -v0a - 1.0, k02 = xv2, k03 = -v0b, k12 = v2a, k13 = gab, k23 = -v2b - 1.0;
-  const double pk = k01 * k23 - k02 * k13 + k03 * k12;
+  const double pk = __fma_rn(k03, k12, __fma_rn(k01, k23, -__dmul_rn(k02, k13)));  // k01 k23 - k02 k13 + k03 k12
   const double ip = 1.0 / pk;
   // K^{-1} = [[0, -k23, k13, -k12], [k23, 0, -k03, k02], [-k13, k03, 0, -k01], [k12, -k02, k01, 0]] / Pf(K)
   const double Ki[4][4] = {{0.0, -k23 * ip, k13 * ip, -k12 * ip},
@@ -503,7 +505,9 @@ __device__ __forceinline__ void warp_skew_update(const DevDims& d, const DevPara
     const int i = lane + 32 * m < N ? lane + 32 * m : N - 1;
     const double vi[4] = {v[i], v[N + i], v[2 * N + i], v[3 * N + i]};
 #pragma unroll
-    for (int q = 0; q < 4; q++) z[m][q] = vi[0] * Ki[0][q] + vi[1] * Ki[1][q] + vi[2] * Ki[2][q] + vi[3] * Ki[3][q];
+    for (int q = 0; q < 4; q++)
+      z[m][q] = __fma_rn(vi[3], Ki[3][q],
+                         __fma_rn(vi[2], Ki[2][q], __fma_rn(vi[0], Ki[0][q], __dmul_rn(vi[1], Ki[1][q]))));
   }
   __syncwarp();
 #pragma unroll
@@ -554,6 +558,12 @@ __host__ __device__ size_t skew_sampler_smem(const DevDims& d, int nwarps, int n
   return off + (size_t)ntile * d.N * (d.N + 1) * 8;
 }
 
+// A chain is the same to the bit whatever the number of blocks and warps that carry it: psi' is summed in one order, and
+// where the compiler could contract a sum of products in more than one way (the exchange ratio, Pf(K), V K^{-1}) the
+// operations are written out.  A last bit matters here: at 4x4 the drift between recomputes reaches the threshold of
+// make_sample.f90:120, and of 3,840 walkers 55 took another decision there when the order of the sum and the contraction
+// followed the block.
+//
 // Bounded by instructions on the SMs that have a walker: with the walker's G in L2 (72 projections of 10 KB at 6x6) a
 // proposal is an x^ . G y^ product per projection, 2,800 warp instructions each before N was a constant.  Measured,
 // make_sample of 64 walkers, 6x6 with translations, 35 sweeps: 104 -> 65 ms with 16 warps, row batches and staged
@@ -621,11 +631,7 @@ __global__ void __launch_bounds__(kSmpThreads, 1)
     if (nacc_tmp > nfastup) {
       fetch_wait();
       ahead = false;
-      if (m.size > 1) {  // the drift measure takes the Pfaffians of all projections
-        m.sync();
-        for (int i = tid; m.own(i) < d.n_qp; i += blockDim.x) m.put(s.pf + m.own(i), s.pf[m.own(i)]);
-      }
-      m.sync();
+      __syncthreads();
       checkpoint<0, 0, F>(c, nfastup, i0);
       if (status(c)) break;
       nacc_tmp = 0;
@@ -658,39 +664,44 @@ __global__ void __launch_bounds__(kSmpThreads, 1)
       __syncthreads();
       cta_rbm_factors(d, s.thp, s.rbm);
       __syncthreads();
-      double pre = 0.0, pim = 0.0;
+      // Pfaffians and amplitudes of the proposal; a block may be one proposal ahead of another, so two sets
+      double* pfn = m.size > 1 ? m.slots + parity * 3 * d.n_qp : s.pfp;
+      double* psn = m.size > 1 ? pfn + d.n_qp : s.psip;
+      parity ^= 1;
       for (int qp = qp0; qp < d.n_qp; qp += qstep) {
         const double R = staged
             ? warp_skew_ratio<N>(d, p, buf, qp, s.idx, i3, i4, ra_new, rb_new, xh, yh, true)
             : warp_skew_ratio<N>(d, p, G0(qp), qp, s.idx, i3, i4, ra_new, rb_new, xh, yh, false);
         if (staged) fetch_tile<N>(buf, G0(qp + qstep < d.n_qp ? qp + qstep : qp0));
         if (lane == 0) {
-          const double pfn = R * s.pf[qp];
-          s.pfp[qp] = pfn;
+          const double pfq = R * s.pf[qp];
           const cplx cw = psi_wo_pf(d, t, s.rbm[qp], s.sgnp[qp >> 1], qp);
-          s.psip[2 * qp] = cw.re * pfn;
-          s.psip[2 * qp + 1] = cw.im * pfn;
-          pre += cw.re * pfn;
-          pim += cw.im * pfn;
+          m.put(pfn + qp, pfq);
+          m.put(psn + 2 * qp, cw.re * pfq);
+          m.put(psn + 2 * qp + 1, cw.im * pfq);
         }
-      }
-      // partial sums of all warps of the walker; a block may be one proposal ahead of another, so two sets of slots
-      double* part = m.size > 1 ? m.slots + 2 * parity * qstep : s.red;
-      parity ^= 1;
-      if (lane == 0) {
-        m.put(part + m.rank * nwarps + warp, pre);
-        m.put(part + (m.size > 1 ? qstep : 32) + m.rank * nwarps + warp, pim);
       }
       m.sync();
+      // psi': one sum for every residue of qp mod 8, then these in order, whatever the number of warps and blocks
+      const double* sums = psn;
+      if (d.n_qp > kPsiSums) {
+        sums = s.red;
+        if (tid < 2 * kPsiSums) {
+          double v = 0.0;
+#pragma unroll 4
+          for (int k = tid; k < 2 * d.n_qp; k += 2 * kPsiSums) v += psn[k];
+          s.red[tid] = v;
+        }
+        if (warp == 0) __syncwarp();
+      }
       if (tid == 0) {
         double re = 0.0, im = 0.0;
-        const double* pi = part + (m.size > 1 ? qstep : 32);
-        const int nsum = m.size > 1 ? qstep : min(nwarps, d.n_qp);  // warps with a projection
-#pragma unroll 4
-        for (int k = 0; k < nsum; k++) {
-          re += part[k];
-          im += pi[k];
-        }
+#pragma unroll
+        for (int k = 0; k < kPsiSums; k++)
+          if (k < d.n_qp) {
+            re += sums[2 * k];
+            im += sums[2 * k + 1];
+          }
         s.dsc[D_PSIPR] = re;
         s.dsc[D_PSIPI] = im;
         (void)grnd(s.mt);  // sub.f90:72
@@ -711,10 +722,10 @@ __global__ void __launch_bounds__(kSmpThreads, 1)
         }
         for (int j = tid; j < d.Mr; j += blockDim.x) s.th[j] = s.thp[j];
         for (int mp = tid; mp < d.n_mp; mp += blockDim.x) s.sgn[mp] = s.sgnp[mp];
-        for (int i = tid, qp; (qp = m.own(i)) < d.n_qp; i += blockDim.x) {
-          s.pf[qp] = s.pfp[qp];
-          s.psi[2 * qp] = s.psip[2 * qp];
-          s.psi[2 * qp + 1] = s.psip[2 * qp + 1];
+        for (int qp = tid; qp < d.n_qp; qp += blockDim.x) {
+          s.pf[qp] = pfn[qp];
+          s.psi[2 * qp] = psn[2 * qp];
+          s.psi[2 * qp + 1] = psn[2 * qp + 1];
         }
         __syncthreads();
         if (tid == 0) {
@@ -1131,7 +1142,7 @@ cudaError_t launch_skew_sampler(const void* kernel, const void* team_kernel, Dev
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   for (; size > 1; size /= 2) {
-    if ((size - 1) * nwarps >= d.n_qp || team_slots(nwarps, size) > 2 * nwarps * d.Np || d.nw * size > nsm)
+    if ((size - 1) * nwarps >= d.n_qp || team_slots(d.n_qp, size) > 2 * nwarps * d.Np || d.nw * size > nsm)
       continue;
     at.val.clusterDim.x = size;
     cfg.gridDim = dim3(d.nw * size);
